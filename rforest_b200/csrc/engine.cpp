@@ -890,16 +890,17 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     }
     if (g.idx.empty()) continue;
     g.crt_high = high != 0;
-    // longest entries first (the warp that gets one works longest), ties in
-    // entry order: one sort of packed (longest-first key, index) integers.
     // (Grouping by prime count first, for instruction-cache locality,
     // measured no better: 11.45 against 11.29 ms on the default step.)
-    std::vector<uint64_t> keys(g.idx.size());
-    for (size_t i = 0; i < keys.size(); ++i)
-      keys[i] = ((uint64_t)(0xffffffffu - inv_[g.idx[i]].out_words) << 32) | g.idx[i];
-    std::sort(keys.begin(), keys.end());
-    for (size_t i = 0; i < keys.size(); ++i) g.idx[i] = (uint32_t)keys[i];
-    rec_groups_.push_back(std::move(g));
+    Group sg;  // entries in segments: launches of their own
+    sg.P = g.P;
+    sg.crt_high = g.crt_high;
+    sg.rmin = g.rmin;
+    sg.crt_off = (uint32_t)crt_items_.size();
+    crt_items(inv_.data(), &g.idx, context().num_sms, &n_recs_, &crt_items_);
+    sg.seg_items = (uint32_t)crt_items_.size() - sg.crt_off;
+    if (sg.seg_items) rec_groups_.push_back(std::move(sg));
+    if (!g.idx.empty()) rec_groups_.push_back(std::move(g));
   }
   for (auto* gs : {&fwd_groups_, &inv_groups_, &rec_groups_})
     for (auto& g : *gs) {
@@ -907,6 +908,10 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
       g.idx_off = (uint32_t)idx_all_.size();
       idx_all_.insert(idx_all_.end(), g.idx.begin(), g.idx.end());
     }
+  // the segments' records follow the residues
+  n_res_ = (n_res_ + 15) & ~(uint64_t)15;
+  off_rec_ = n_res_;
+  n_res_ += (uint64_t)n_recs_ * (sizeof(CrtRec) / sizeof(uint32_t));
   prepared_ = true;
   return kOk;
 }
@@ -925,7 +930,8 @@ int Plan::bind(Workspace* ws) {
   off_tc_ = align16(off_items_ + items_.size() * sizeof(ContractItem));
   off_idx_ = align16(off_tc_ + tc_items_.size() * sizeof(ContractItem));
   off_cta_ = align16(off_idx_ + idx_all_.size() * sizeof(uint32_t));
-  desc_bytes_ = align16(off_cta_ + cta_items_.size() * sizeof(CtaItem));
+  off_crt_ = align16(off_cta_ + cta_items_.size() * sizeof(CtaItem));
+  desc_bytes_ = align16(off_crt_ + crt_items_.size() * sizeof(CrtItem));
   plan_transfers();
   ws_ = ws ? ws : &own_;
   int st = ws_->reserve(n_limbs_, n_res_, n_out_words_, outs_.size(), desc_bytes_, stage_limbs_,
@@ -943,6 +949,8 @@ int Plan::bind(Workspace* ws) {
     std::memcpy(hd + off_idx_, idx_all_.data(), idx_all_.size() * sizeof(uint32_t));
   if (!cta_items_.empty())
     std::memcpy(hd + off_cta_, cta_items_.data(), cta_items_.size() * sizeof(CtaItem));
+  if (!crt_items_.empty())
+    std::memcpy(hd + off_crt_, crt_items_.data(), crt_items_.size() * sizeof(CrtItem));
   d_fwd_ = reinterpret_cast<FwdDesc*>(ws_->d_desc + off_fwd_);
   d_inv_ = reinterpret_cast<InvDesc*>(ws_->d_desc + off_inv_);
   d_pd_ = reinterpret_cast<ProdDesc*>(ws_->d_desc + off_pd_);
@@ -950,6 +958,7 @@ int Plan::bind(Workspace* ws) {
   d_tc_items_ = reinterpret_cast<ContractItem*>(ws_->d_desc + off_tc_);
   d_idx_ = reinterpret_cast<uint32_t*>(ws_->d_desc + off_idx_);
   d_cta_ = reinterpret_cast<CtaItem*>(ws_->d_desc + off_cta_);
+  d_crt_ = reinterpret_cast<CrtItem*>(ws_->d_desc + off_crt_);
   int64_t sl[kStages];
   stage_launches(sl);
   launches_ = sl[0] + sl[1] + sl[2] + sl[3];
@@ -1249,8 +1258,9 @@ int Plan::launch_all(cudaStream_t st, bool timed) {
   if (timed) CU(cudaEventRecord(ev[3], st), "cudaEventRecord");
   r = fan_out(ws_, st, (int)rec_groups_.size(), [&](int i, cudaStream_t s) -> int {
     const Group& g = rec_groups_[i];
-    CU(launch_crt_mixed(d_inv_, d_idx_ + g.idx_off, (int)g.idx.size(), g.crt_high, g.rmin.data(),
-                        ws_->d_res, ws_->d_out, ws_->d_sizes, s),
+    CU(launch_crt_mixed(d_inv_, d_crt_ + g.crt_off, (int)g.seg_items, d_idx_ + g.idx_off,
+                        (int)g.idx.size(), g.crt_high, g.rmin.data(), ws_->d_res, ws_->d_out,
+                        ws_->d_sizes, reinterpret_cast<CrtRec*>(ws_->d_res + off_rec_), s),
        "CRT+recompose launch");
     return kOk;
   });
@@ -1288,7 +1298,8 @@ void Plan::stage_launches(int64_t out[kStages]) const {
   out[0] = count(fwd_groups_);
   out[1] = (items_.empty() ? 0 : 1) + (tc_items_.empty() ? 0 : 1);
   out[2] = count(inv_groups_);
-  out[3] = (int64_t)rec_groups_.size();
+  out[3] = 0;
+  for (const Group& g : rec_groups_) out[3] += g.seg_items ? kCrtSegLaunches : 1;
 }
 
 int Plan::download_enqueue(cudaStream_t st) {

@@ -322,6 +322,7 @@ class Plan {
     // narrowest coefficient width per count
     bool crt_high = false;
     std::vector<int> rmin;
+    uint32_t crt_off = 0, seg_items = 0;  // its segments (crt_items)
   };
 
   std::vector<ProductSpec> prods_;
@@ -335,6 +336,9 @@ class Plan {
   std::vector<Group> fwd_groups_, inv_groups_, rec_groups_;
   std::vector<uint32_t> idx_all_;
   std::vector<CtaItem> cta_items_;
+  std::vector<CrtItem> crt_items_;
+  uint32_t n_recs_ = 0;    // segment records of the CRT, kept behind the residues
+  uint64_t off_rec_ = 0;   // first residue word of them
   std::vector<OutRef> outs_;          // flattened output references
   std::vector<int64_t> out_word_off_; // per output entry (words)
   std::vector<int32_t> out_limbs_;    // per output entry: limbs the device writes
@@ -377,8 +381,9 @@ class Plan {
   Workspace* ws_ = nullptr;
   // descriptor blob: offsets of each section (bytes) and its size
   size_t off_fwd_ = 0, off_inv_ = 0, off_pd_ = 0, off_items_ = 0, off_idx_ = 0, off_cta_ = 0,
-         desc_bytes_ = 0;
+         off_crt_ = 0, desc_bytes_ = 0;
   CtaItem* d_cta_ = nullptr;
+  CrtItem* d_crt_ = nullptr;
   FwdDesc* d_fwd_ = nullptr;
   InvDesc* d_inv_ = nullptr;
   ProdDesc* d_pd_ = nullptr;

@@ -13,9 +13,10 @@
 //   k_crt_mixed      explicit CRT to signed multi-word coefficients, then
 //                    sum_i c_i 2^(i r) with carries resolved by a
 //                    carry-lookahead prefix scan over 32-bit output words,
-//                    sign + negation + normalisation (one warp per entry,
-//                    every prime count of a range in one launch);
-//                    k_crt_warp the same for one prime count
+//                    sign + negation + normalisation (one warp per entry
+//                    or, of few long entries, per segment; every prime
+//                    count of a range in one launch); k_crt_finish closes
+//                    the entries in segments
 //
 // Reference counterparts: split/reduce src/lib/split_reduce.c:15-66,
 // NTTs src/lib/mpnfft.c:354-432, contraction src/lib/mpnfft.c:559-651,
@@ -24,8 +25,10 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <vector>
 
 #include "kernels.h"
 #include "modarith.cuh"
@@ -1034,7 +1037,8 @@ k_inv_cols(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx, 
 
 
 // ---------------------------------------------------------------------------
-// CRT + recompose, one warp per output entry (no block barriers).
+// CRT + recompose, one warp per output entry or segment of one (no block
+// barriers).
 //
 // Explicit CRT (crt_coeff) to the symmetric P-word value U_i - s_i 2^(32P)
 // of each coefficient (s_i = top bit of U_i), per-word gathered sums, carries
@@ -1046,6 +1050,7 @@ k_inv_cols(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx, 
 constexpr int kCrtWarps = 4;       // entries per CTA
 constexpr int kCrtSteps = 8;       // 32-word steps per tile
 constexpr int kCrtTileWords = 32 * kCrtSteps;
+constexpr size_t kCrtSmemLimit = 200 * 1024;
 
 // Explicit CRT of one coefficient (constants in CrtConst): the symmetric
 // residue X in (-M_P/4, M_P/4) as P words of two's complement.
@@ -1124,31 +1129,73 @@ struct FastDiv {
   }
 };
 
-// One output entry by one warp: CRT of its coefficients tile by tile into
-// the warp's scratch sV, each coefficient pre-shifted to its place in the
-// output words (P + 1 words of tile coefficient c at [c (P + 1)]), the
-// words' sums, the carry ripple, the sign and the size.
-template <int P>
-__device__ __forceinline__ void crt_entry(const InvDesc& d, const uint32_t* __restrict__ res,
+// The carry into word `wbeg` of a segment, from a look at the 32 words below
+// it (lane l holds word wbeg - 32 + l; lane 0 lacks the word below it, so
+// its own carry stays open): kTfUnknown when every word of 1..31 lets a
+// carry pass.
+constexpr int kCarryUnknown = 2;
+__device__ __forceinline__ bool tf_const(uint32_t f) {
+  return ((f ^ (f >> 2)) & 15u) == 0u;
+}
+__device__ __forceinline__ int lookback_carry(uint32_t y, int g, bool prop, int lane) {
+  const unsigned FULL = 0xffffffffu;
+  const unsigned pm = __ballot_sync(FULL, prop);
+  if (!(pm >> 31)) return __shfl_sync(FULL, g, 31);  // word wbeg - 1 settles it
+  uint32_t inc = lane == 0 ? kTfIdentity : word_tf(y, g);
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t u = __shfl_up_sync(FULL, inc, off);
+    if (lane >= off) inc = compose_tf(inc, u);
+  }
+  inc = __shfl_sync(FULL, inc, 31);
+  return tf_const(inc) ? apply_tf(inc, 0) : kCarryUnknown;
+}
+
+// Words [wbeg, wend) of one output entry by one warp: CRT of its
+// coefficients tile by tile into the warp's scratch sV, each coefficient
+// pre-shifted to its place in the output words (P + 1 words of tile
+// coefficient c at [c (P + 1)]), the words' sums, the carry ripple.
+//
+// SEG false: the whole entry (wbeg = 0, wend = out_words), with its sign,
+// negation and size.  SEG true: one segment of an entry that several warps
+// share (wbeg a multiple of 32): the carry into the segment comes from
+// the 32 words below it, which the first tile computes again without
+// storing them; the words are written in two's complement and the record
+// tells k_crt_finish what it needs of the segment.  While the carry in is
+// unknown (the words below are all 0 or all ones: structured operands, or
+// the sign fill above a short result) the words are written for a carry of
+// 0 and the record keeps the three possible outcomes.
+//
+// One warp an entry, whatever its length, left the GPU idle on few long
+// entries: a 2 x 2 product of 10^7-bit integers spent 12.9 of its 13.3 ms on
+// four warps here, an 8 x 8 one of 2^16-bit integers 103 of 150 us of
+// kernels on 64.  (Two kernels, because the segment's state costs whole
+// entries 8 registers and a CTA less an SM: 9 % of the stage's time.)
+template <int P, bool SEG>
+__device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* __restrict__ res,
                                           uint32_t* __restrict__ out,
                                           int32_t* __restrict__ out_sizes, uint32_t* sV,
-                                          int cmax, int lane) {
+                                          int wbeg, int wend, CrtRec* __restrict__ rec,
+                                          int lane) {
   const unsigned FULL = 0xffffffffu;
   // bit positions fit 31 bits (an entry's words times 32 stays below 2^31),
   // so index arithmetic is 32-bit and the divisions by r are multiply-highs
   const int r = (int)d.r;
   const FastDiv divr((uint32_t)r);
-  const int W = (int)d.out_words;
   const int ncoef = (int)d.ncoef;
   uint32_t* o = out + d.out_word;
 
   int hi_prev = 0, carry = 0;
   int first_nz = 0x7fffffff, last_nz = -1, last_no = -1;
   uint32_t topval = 0;
-  for (int w0 = 0; w0 < W; w0 += kCrtTileWords) {
+  bool unknown = false;           // the carry into the segment is still open
+  bool open = false, top_open = false;  // it was at the start / at the last step
+  uint32_t cf = kTfIdentity;      // from that carry to the current one
+  for (int w0 = SEG && wbeg > 0 ? wbeg - 32 : 0; w0 < wend; w0 += kCrtTileWords) {
+    const int wt = w0 + kCrtTileWords < wend ? w0 + kCrtTileWords : wend;
     int lo_i = 0;
     if (32 * w0 > 32 * P) lo_i = (int)divr((uint32_t)(32 * w0 - 32 * P + r - 1));
-    int hi_i = (int)divr((uint32_t)(32 * (w0 + kCrtTileWords) - 1));
+    int hi_i = (int)divr((uint32_t)(32 * wt - 1));
     if (hi_i > ncoef - 1) hi_i = ncoef - 1;
     const int ncf = hi_i >= lo_i ? hi_i - lo_i + 1 : 0;
     // coefficient i = lo_i + c as X_i 2^(i r mod 32): P + 1 words, the top
@@ -1170,8 +1217,10 @@ __device__ __forceinline__ void crt_entry(const InvDesc& d, const uint32_t* __re
     }
     __syncwarp();
     for (int st = 0; st < kCrtSteps; ++st) {
-      const int w = w0 + st * 32 + lane;
-      const bool active = w < W;
+      const int ws = w0 + 32 * st;
+      if (ws >= wt) break;
+      const int w = ws + lane;
+      const bool active = w < wend;
       int64_t sw = 0;
       if (active) {
         int ia = lo_i;
@@ -1191,12 +1240,26 @@ __device__ __forceinline__ void crt_entry(const InvDesc& d, const uint32_t* __re
       const int hi = active ? (int)(sw >> 32) : 0;
       int hprev = __shfl_up_sync(FULL, hi, 1);
       if (lane == 0) hprev = hi_prev;
+      hi_prev = __shfl_sync(FULL, hi, 31);
       const int64_t z = (int64_t)(uint32_t)sw + hprev;
       const uint32_t y = (uint32_t)z;
       const int g = active ? (int)(z >> 32) : 0;
       const bool prop = active && (y == 0u || y == 0xffffffffu);
+      if (SEG && ws < wbeg) {  // the look at the words below the segment
+        carry = lookback_carry(y, g, prop, lane);
+        if (carry == kCarryUnknown) {
+          unknown = open = true;
+          carry = 0;
+          if (lane == 0)
+            for (int c = 0; c < 3; ++c) {
+              rec->first_nz[c] = 0x7fffffff;
+              rec->last_nz[c] = rec->last_no[c] = -1;
+            }
+        }
+        continue;
+      }
       int cin, cout;
-      if (__any_sync(FULL, prop)) {
+      if (__any_sync(FULL, prop) || (SEG && unknown)) {
         const uint32_t f = active ? word_tf(y, g) : kTfIdentity;
         uint32_t inc = f;
 #pragma unroll
@@ -1206,8 +1269,24 @@ __device__ __forceinline__ void crt_entry(const InvDesc& d, const uint32_t* __re
         }
         uint32_t exc = __shfl_up_sync(FULL, inc, 1);
         if (lane == 0) exc = kTfIdentity;
+        const uint32_t all = __shfl_sync(FULL, inc, 31);
+        if (SEG && unknown) {  // this step's outcomes for each carry into the segment
+          for (int c = 0; c < 3; ++c) {
+            const uint32_t F = y + (uint32_t)apply_tf(compose_tf(exc, cf), c - 1);
+            const unsigned nz = __ballot_sync(FULL, active && F != 0u);
+            const unsigned no = __ballot_sync(FULL, active && F != 0xffffffffu);
+            const unsigned top = __ballot_sync(FULL, w == wend - 1 && (F >> 31));
+            if (lane == 0) {
+              if (nz && rec->first_nz[c] == 0x7fffffff) rec->first_nz[c] = ws + __ffs(nz) - 1;
+              if (nz) rec->last_nz[c] = ws + 31 - __clz(nz);
+              if (no) rec->last_no[c] = ws + 31 - __clz(no);
+              rec->top[c] = top != 0;
+            }
+          }
+          cf = compose_tf(all, cf);
+        }
         cin = apply_tf(exc, carry);
-        cout = apply_tf(__shfl_sync(FULL, inc, 31), carry);
+        cout = apply_tf(all, carry);
       } else {
         cin = __shfl_up_sync(FULL, g, 1);
         if (lane == 0) cin = carry;
@@ -1216,15 +1295,20 @@ __device__ __forceinline__ void crt_entry(const InvDesc& d, const uint32_t* __re
       if (active) {
         const uint32_t F = y + (uint32_t)cin;
         o[w] = F;
-        if (F != 0u) {
-          if ((int)w < first_nz) first_nz = (int)w;
-          last_nz = (int)w;
+        if (!SEG || !unknown) {
+          if (F != 0u) {
+            if (w < first_nz) first_nz = w;
+            last_nz = w;
+          }
+          if (F != 0xffffffffu) last_no = w;
+          if (w == wend - 1) topval = F;
         }
-        if (F != 0xffffffffu) last_no = (int)w;
-        if (w == W - 1) topval = F;
       }
-      hi_prev = __shfl_sync(FULL, hi, 31);
       carry = cout;
+      if (SEG) {
+        top_open = unknown;
+        if (unknown && tf_const(cf)) unknown = false;  // settled from the next word on
+      }
     }
     __syncwarp();
   }
@@ -1232,11 +1316,29 @@ __device__ __forceinline__ void crt_entry(const InvDesc& d, const uint32_t* __re
   last_nz = __reduce_max_sync(FULL, last_nz);
   last_no = __reduce_max_sync(FULL, last_no);
   topval = __reduce_or_sync(FULL, topval);
-  const bool negative = W > 0 && (topval >> 31);
+  if (SEG) {
+    if (lane != 0) return;
+    for (int c = 0; c < 3; ++c) {
+      if (!open) {
+        rec->first_nz[c] = first_nz;
+        rec->last_nz[c] = last_nz;
+        rec->last_no[c] = last_no;
+      } else {
+        rec->first_nz[c] = min(rec->first_nz[c], first_nz);
+        rec->last_nz[c] = max(rec->last_nz[c], last_nz);
+        rec->last_no[c] = max(rec->last_no[c], last_no);
+      }
+      if (!top_open) rec->top[c] = (int32_t)(topval >> 31);
+    }
+    rec->tf = unknown ? cf : 0x15u * (uint32_t)(carry + 1);
+    rec->open = open;
+    return;
+  }
+  const bool negative = wend > 0 && (topval >> 31);
   int top;
   if (negative) {
     const int zf = first_nz;
-    for (int64_t w = zf + lane; w < W; w += 32) {
+    for (int w = zf + lane; w < wend; w += 32) {
       const uint32_t F = o[w];
       o[w] = (w == zf) ? (0u - F) : ~F;
     }
@@ -1250,48 +1352,136 @@ __device__ __forceinline__ void crt_entry(const InvDesc& d, const uint32_t* __re
   }
 }
 
-// One prime count per launch.
-template <int P>
-__global__ void __launch_bounds__(32 * kCrtWarps)
-k_crt_warp(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx, int count,
-           const uint32_t* __restrict__ res, uint32_t* __restrict__ out,
-           int32_t* __restrict__ out_sizes, int cmax) {
-  extern __shared__ uint32_t sm[];
-  const int warp = threadIdx.x >> 5;
-  const int slot = blockIdx.x * kCrtWarps + warp;
-  if (slot >= count) return;  // whole warp; no block-wide barrier below
-  const InvDesc d = descs[idx[slot]];
-  crt_entry<P>(d, res, out, out_sizes, sm + warp * (cmax * (P + 1)), cmax, threadIdx.x & 31);
+// item `slot` of a launch whose entries 0, 1, ... are all alike
+__device__ __forceinline__ CrtItem uniform_item(const CrtUniform& u, uint32_t slot) {
+  CrtItem it;
+  it.inv = slot / u.nseg;
+  it.seg = slot - it.inv * u.nseg;
+  it.nseg = u.nseg;
+  it.rec = it.inv * u.nseg;
+  it.w0 = it.seg * u.step;
+  it.w1 = it.seg + 1 < u.nseg ? it.w0 + u.step : u.words;
+  return it;
 }
 
-template <int P, int PHI>
-__device__ __forceinline__ void crt_dispatch(const InvDesc& d, const uint32_t* __restrict__ res,
+template <int P, int PHI, bool SEG>
+__device__ __forceinline__ void crt_dispatch(const InvDesc& d, const CrtItem& it,
+                                             const uint32_t* __restrict__ res,
                                              uint32_t* __restrict__ out,
                                              int32_t* __restrict__ out_sizes, uint32_t* sU,
-                                             const CrtScratch& cs, int lane) {
+                                             CrtRec* __restrict__ rec, int lane) {
   if (d.P == P) {
-    crt_entry<P>(d, res, out, out_sizes, sU, cs.cmax[P], lane);
+    crt_range<P, SEG>(d, res, out, out_sizes, sU, (int)it.w0, (int)it.w1, rec, lane);
   } else {
-    if constexpr (P < PHI) crt_dispatch<P + 1, PHI>(d, res, out, out_sizes, sU, cs, lane);
+    if constexpr (P < PHI)
+      crt_dispatch<P + 1, PHI, SEG>(d, it, res, out, out_sizes, sU, rec, lane);
   }
 }
 
-// Prime counts PLO..PHI in one launch (the entries longest first across
-// them, so the long entries of every count start together and the launch
-// has one tail instead of one per count); each warp's scratch holds
-// cs.warp_words words.
-template <int PLO, int PHI>
+// Prime counts PLO..PHI in one launch, one warp an item, longest first across
+// the counts (the launch has one tail instead of one per count): segments
+// (SEG; segs, or u where all entries are alike), or whole entries (idx, or
+// entries 0, 1, ...).  Each warp's scratch holds warp_words words.
+template <int PLO, int PHI, bool SEG>
 __global__ void __launch_bounds__(32 * kCrtWarps)
-k_crt_mixed(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx, int count,
+k_crt_mixed(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs,
+            const uint32_t* __restrict__ idx, int count, CrtUniform u,
             const uint32_t* __restrict__ res, uint32_t* __restrict__ out,
-            int32_t* __restrict__ out_sizes, CrtScratch cs) {
+            int32_t* __restrict__ out_sizes, CrtRec* __restrict__ recs, int warp_words) {
   extern __shared__ uint32_t sm[];
   const int warp = threadIdx.x >> 5;
   const int slot = blockIdx.x * kCrtWarps + warp;
   if (slot >= count) return;  // whole warp; no block-wide barrier below
-  const InvDesc d = descs[idx[slot]];
-  crt_dispatch<PLO, PHI>(d, res, out, out_sizes, sm + warp * cs.warp_words, cs,
-                         threadIdx.x & 31);
+  CrtItem it;
+  if (SEG) {
+    it = segs ? segs[slot] : uniform_item(u, (uint32_t)slot);
+  } else {
+    it.inv = idx ? idx[slot] : (uint32_t)slot;
+    it.w0 = it.rec = it.seg = 0;
+    it.w1 = descs[it.inv].out_words;
+  }
+  const InvDesc d = descs[it.inv];
+  crt_dispatch<PLO, PHI, SEG>(d, it, res, out, out_sizes, sm + warp * warp_words,
+                              SEG ? recs + it.rec + it.seg : nullptr, threadIdx.x & 31);
+}
+
+// The sign, negation and size of entries in segments, one warp a segment:
+// settles the carry into segments whose own look left it open, complements
+// the words of negative entries and (the top segment's warp) writes the
+// size.  Mostly three records tell everything: this segment's carry is
+// known, the one below holds a nonzero word, the top one knows its sign.
+// Otherwise (zeros, powers of two, sign fill above a short result) the warp
+// runs over the entry's records once, 32 a step.
+__global__ void __launch_bounds__(32 * kCrtWarps)
+k_crt_finish(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs, int count,
+             CrtUniform un, const CrtRec* __restrict__ recs, uint32_t* __restrict__ out,
+             int32_t* __restrict__ out_sizes) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int slot = blockIdx.x * kCrtWarps + (threadIdx.x >> 5);
+  if (slot >= count) return;  // whole warp
+  const CrtItem it = segs ? segs[slot] : uniform_item(un, (uint32_t)slot);
+  const InvDesc& d = descs[it.inv];
+  const CrtRec* __restrict__ R = recs + it.rec;
+  const int s = (int)it.seg, S = (int)it.nseg;
+  const CrtRec& me = R[s];
+  uint32_t* o = out + d.out_word;
+  const bool open = me.open != 0;
+  int cs = 1;        // the carry into this segment, plus one
+  bool negative, below;  // the entry's sign; a nonzero word below this segment
+  int top;           // (top segment) last word of the magnitude that is not zero
+  if (!open && !R[S - 1].open && (s == 0 || (!R[s - 1].open && R[s - 1].last_nz[1] >= 0)) &&
+      (s != S - 1 || (me.last_nz[1] >= 0 && me.last_no[1] >= 0))) {
+    negative = R[S - 1].top[1] != 0;
+    below = s > 0;
+    top = negative ? me.last_no[1] : me.last_nz[1];
+  } else {
+    int c = 1, zf = 0x7fffffff, zb = 0x7fffffff, lz = -1, lo = -1, neg = 0;
+    for (int t0 = 0; t0 < S; t0 += 32) {
+      const int t = t0 + lane;
+      const bool live = t < S;
+      const uint32_t tf = live ? R[t].tf : kTfIdentity;
+      int mc = 1;
+#pragma unroll
+      for (int u = 0; u < 32; ++u) {
+        if (lane == u) mc = c;
+        c = (int)((__shfl_sync(FULL, tf, u) >> (2 * c)) & 3u);
+      }
+      const int fn = live ? R[t].first_nz[mc] : 0x7fffffff;
+      zf = min(zf, __reduce_min_sync(FULL, fn));
+      zb = min(zb, __reduce_min_sync(FULL, t < s ? fn : 0x7fffffff));
+      lz = max(lz, __reduce_max_sync(FULL, live ? R[t].last_nz[mc] : -1));
+      lo = max(lo, __reduce_max_sync(FULL, live ? R[t].last_no[mc] : -1));
+      neg |= __reduce_max_sync(FULL, t == S - 1 ? R[t].top[mc] : 0);
+      if (s >= t0 && s < t0 + 32) cs = __shfl_sync(FULL, mc, s - t0);
+    }
+    negative = neg != 0;
+    below = zb != 0x7fffffff;
+    top = negative ? (lo > zf ? lo : zf) : lz;
+  }
+  const int w0 = (int)it.w0, w1 = (int)it.w1;
+  if (open && cs != 1) {  // written for a carry of 0: add it to the segment
+    const uint32_t pass = cs == 2 ? 0xffffffffu : 0u;
+    for (int ws = w0; ws < w1; ws += 32) {
+      const int w = ws + lane;
+      const uint32_t F = w < w1 ? o[w] : pass;
+      const unsigned stop = __ballot_sync(FULL, F != pass);
+      const int k = stop ? __ffs(stop) - 1 : 32;
+      if (w < w1 && lane <= k) o[w] = F + (uint32_t)(cs - 1);
+      if (stop) break;
+    }
+  }
+  if (negative) {
+    const int zf = below ? -1 : me.first_nz[cs];
+    for (int w = w0 + lane; w < w1; w += 32) {
+      const uint32_t F = o[w];
+      if (w >= zf) o[w] = w == zf ? 0u - F : ~F;
+    }
+  }
+  if (s == S - 1 && lane == 0) {
+    const int limbs = top >= 0 ? top / 2 + 1 : 0;
+    out_sizes[d.entry] = negative ? -limbs : limbs;
+  }
 }
 
 
@@ -2156,75 +2346,112 @@ static int crt_cmax(int P, int rmin) {
   return (int)((32 * (int64_t)kCrtTileWords + 32 * P) / rmin + 3);
 }
 
-cudaError_t launch_crt_mixed(const InvDesc* descs, const uint32_t* idx, int count, bool high,
-                             const int* rmin, const uint32_t* res, uint32_t* out, int32_t* sizes,
+// Words a warp takes of an entry when a launch writes total_words words: as
+// many as leave every SM kCrtSegWarps warps (a little over two waves of
+// them, so that no long entry is the launch's tail), in whole tiles less the
+// 32 words of the look below a segment.
+constexpr int kCrtSegWarps = 64;
+static int crt_segment_words(uint64_t total_words, int sms) {
+  const uint64_t t = total_words / ((uint64_t)(sms > 0 ? sms : 1) * kCrtSegWarps);
+  const uint64_t tiles = (t + 32 + kCrtTileWords - 1) / kCrtTileWords;
+  return (int)((tiles < 1 ? 1 : tiles) * kCrtTileWords) - 32;
+}
+
+// Segments of an entry of W words, each *step words but the last.  The look
+// and the second launch cost a segment about 40 words' time, so an entry of
+// up to two segments stays whole, and where a warp an entry fills the SMs
+// only entries well above the others are split (4096 entries of 2050 words
+// took 121 us whole, 140 in five segments; 2000 of 630 words 33 and 38; 256
+// mixed products 950 us with the long entries split, 1000 without).
+constexpr uint32_t kCrtShort = 16 * kCrtTileWords;
+static uint32_t crt_split(uint32_t W, uint32_t seg, bool few, uint32_t* step) {
+  const bool split = few ? W > 2 * seg : W > kCrtShort && W > 3 * seg;
+  uint32_t ns = split ? (W + seg - 1) / seg : 1u;
+  *step = (((W + ns - 1) / ns) + 31) & ~31u;
+  return ns > 1 ? (W + *step - 1) / *step : 1u;
+}
+static bool crt_few(uint64_t count, int sms) { return count < 8 * (uint64_t)sms; }
+
+CrtUniform crt_uniform(uint32_t words, uint32_t count, int sms, uint64_t max_recs) {
+  CrtUniform u;
+  u.words = words;
+  u.nseg = crt_split(words, (uint32_t)crt_segment_words((uint64_t)words * count, sms),
+                     crt_few(count, sms), &u.step);
+  if ((uint64_t)u.nseg * count > max_recs) u.nseg = 1;
+  return u;
+}
+
+void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, uint32_t* nrecs,
+               std::vector<CrtItem>* segs) {
+  // longest entries first (the warp that gets one works longest), ties in
+  // entry order: one sort of packed (longest-first key, index) integers,
+  // which the entries of a single product need not
+  std::vector<uint64_t> keys(idx->size());
+  uint64_t total = 0;
+  for (size_t i = 0; i < keys.size(); ++i) {
+    const uint32_t W = descs[(*idx)[i]].out_words;
+    total += W;
+    keys[i] = ((uint64_t)(0xffffffffu - W) << 32) | (*idx)[i];
+  }
+  if (!std::is_sorted(keys.begin(), keys.end())) std::sort(keys.begin(), keys.end());
+  const uint32_t seg = (uint32_t)crt_segment_words(total, sms);
+  const bool few = crt_few(keys.size(), sms);
+  idx->clear();
+  for (const uint64_t key : keys) {
+    const uint32_t e = (uint32_t)key, W = descs[e].out_words;
+    uint32_t step;
+    const uint32_t ns = crt_split(W, seg, few, &step);
+    if (ns == 1) {
+      idx->push_back(e);
+      continue;
+    }
+    for (uint32_t s = 0; s < ns; ++s)
+      segs->push_back(CrtItem{e, s * step, s + 1 < ns ? (s + 1) * step : W, *nrecs, s, ns});
+    *nrecs += ns;
+  }
+}
+
+template <int PLO, int PHI>
+static cudaError_t launch_crt(const InvDesc* descs, const CrtItem* segs, int nsegs,
+                              const uint32_t* idx, int count, CrtUniform u, int warp_words,
+                              const uint32_t* res, uint32_t* out, int32_t* sizes, CrtRec* recs,
+                              cudaStream_t st) {
+  const size_t smem = sizeof(uint32_t) * (size_t)warp_words * kCrtWarps;
+  if (smem == 0 || smem > kCrtSmemLimit) return cudaErrorInvalidValue;
+  constexpr int NT = 32 * kCrtWarps;
+  const int gs = (nsegs + kCrtWarps - 1) / kCrtWarps, gw = (count + kCrtWarps - 1) / kCrtWarps;
+  if (nsegs > 0) {
+    k_crt_mixed<PLO, PHI, true><<<gs, NT, smem, st>>>(descs, segs, nullptr, nsegs, u, res, out,
+                                                      sizes, recs, warp_words);
+    k_crt_finish<<<gs, NT, 0, st>>>(descs, segs, nsegs, u, recs, out, sizes);
+  }
+  if (count > 0)
+    k_crt_mixed<PLO, PHI, false><<<gw, NT, smem, st>>>(descs, nullptr, idx, count, u, res, out,
+                                                       sizes, recs, warp_words);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_crt_mixed(const InvDesc* descs, const CrtItem* segs, int nsegs,
+                             const uint32_t* idx, int count, bool high, const int* rmin,
+                             const uint32_t* res, uint32_t* out, int32_t* sizes, CrtRec* recs,
                              cudaStream_t st) {
-  if (count == 0) return cudaSuccess;
   const int plo = high ? kCrtMixedSplit + 1 : 2, phi = high ? kMaxPrimes : kCrtMixedSplit;
-  CrtScratch cs;
-  cs.warp_words = 0;
-  for (int P = 0; P <= kMaxPrimes; ++P) {
-    cs.cmax[P] = 0;
-    if (P < plo || P > phi || rmin[P] <= 0) continue;
-    cs.cmax[P] = crt_cmax(P, rmin[P]);
-    if (cs.cmax[P] * (P + 1) > cs.warp_words) cs.warp_words = cs.cmax[P] * (P + 1);
-  }
-  if (cs.warp_words == 0) return cudaErrorInvalidValue;
-  const size_t smem = sizeof(uint32_t) * (size_t)cs.warp_words * kCrtWarps;
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  const int grid = (count + kCrtWarps - 1) / kCrtWarps;
-  if (high)
-    k_crt_mixed<kCrtMixedSplit + 1, kMaxPrimes><<<grid, 32 * kCrtWarps, smem, st>>>(
-        descs, idx, count, res, out, sizes, cs);
-  else
-    k_crt_mixed<2, kCrtMixedSplit><<<grid, 32 * kCrtWarps, smem, st>>>(descs, idx, count, res,
-                                                                      out, sizes, cs);
-  return cudaGetLastError();
+  int words = 0;
+  for (int P = plo; P <= phi; ++P)
+    if (rmin[P] > 0) words = std::max(words, crt_cmax(P, rmin[P]) * (P + 1));
+  const auto fn = high ? launch_crt<kCrtMixedSplit + 1, kMaxPrimes> : launch_crt<2, kCrtMixedSplit>;
+  return fn(descs, segs, nsegs, idx, count, CrtUniform{}, words, res, out, sizes, recs, st);
 }
 
-template <int P>
-static cudaError_t launch_crt_t(const InvDesc* descs, const uint32_t* idx, int count,
-                                const uint32_t* res, uint32_t* out, int32_t* sizes, int rmin,
-                                cudaStream_t st) {
-  const int cmax = crt_cmax(P, rmin);
-  const size_t per_warp = sizeof(uint32_t) * (size_t)(cmax * (P + 1));
-  const size_t smem = per_warp * kCrtWarps;
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  const int grid = (count + kCrtWarps - 1) / kCrtWarps;
-  k_crt_warp<P><<<grid, 32 * kCrtWarps, smem, st>>>(descs, idx, count, res, out, sizes, cmax);
-  return cudaGetLastError();
+cudaError_t launch_crt_uniform(const InvDesc* descs, int count, CrtUniform u, int P, int r,
+                               const uint32_t* res, uint32_t* out, int32_t* sizes, CrtRec* recs,
+                               cudaStream_t st) {
+  const bool seg = u.nseg > 1;
+  const auto fn = P > kCrtMixedSplit ? launch_crt<kCrtMixedSplit + 1, kMaxPrimes>
+                                     : launch_crt<2, kCrtMixedSplit>;
+  return fn(descs, nullptr, seg ? count * (int)u.nseg : 0, nullptr, seg ? 0 : count, u,
+            crt_cmax(P, r) * (P + 1), res, out, sizes, recs, st);
 }
-
-cudaError_t launch_crt_recompose(const InvDesc* descs, const uint32_t* idx, int count, int P,
-                                 const uint32_t* res, uint32_t* out, int32_t* sizes, int rmin,
-                                 cudaStream_t st) {
-  if (count == 0) return cudaSuccess;
-  if (rmin < 1) return cudaErrorInvalidValue;
-  switch (P) {
-#define MPZMM_CRT_CASE(PP) \
-  case PP:                 \
-    return launch_crt_t<PP>(descs, idx, count, res, out, sizes, rmin, st);
-    MPZMM_CRT_CASE(2)
-    MPZMM_CRT_CASE(3)
-    MPZMM_CRT_CASE(4)
-    MPZMM_CRT_CASE(5)
-    MPZMM_CRT_CASE(6)
-    MPZMM_CRT_CASE(7)
-    MPZMM_CRT_CASE(8)
-    MPZMM_CRT_CASE(9)
-    MPZMM_CRT_CASE(10)
-    MPZMM_CRT_CASE(11)
-    MPZMM_CRT_CASE(12)
-    MPZMM_CRT_CASE(13)
-    MPZMM_CRT_CASE(14)
-    MPZMM_CRT_CASE(15)
-    MPZMM_CRT_CASE(16)
-#undef MPZMM_CRT_CASE
-    default:
-      return cudaErrorInvalidValue;
-  }
-}
-
 
 // Dynamic shared memory limits of every kernel, set once per device at
 // set-up (so that launches, including those captured into a CUDA graph,
@@ -2240,12 +2467,6 @@ static cudaError_t set_fwd_attrs() {
         cudaSuccess)
       return e;
   return cudaSuccess;
-}
-
-template <int P>
-static cudaError_t set_crt_attr() {
-  return cudaFuncSetAttribute(k_crt_warp<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              200 * 1024);
 }
 
 cudaError_t init_kernel_attributes() {
@@ -2269,22 +2490,12 @@ cudaError_t init_kernel_attributes() {
       (e = set_fwd_attrs<5>()) != cudaSuccess || (e = set_fwd_attrs<6>()) != cudaSuccess ||
       (e = set_fwd_attrs<7>()) != cudaSuccess)
     return e;
-  if ((e = set_crt_attr<2>()) != cudaSuccess || (e = set_crt_attr<3>()) != cudaSuccess ||
-      (e = set_crt_attr<4>()) != cudaSuccess || (e = set_crt_attr<5>()) != cudaSuccess ||
-      (e = set_crt_attr<6>()) != cudaSuccess || (e = set_crt_attr<7>()) != cudaSuccess ||
-      (e = set_crt_attr<8>()) != cudaSuccess || (e = set_crt_attr<9>()) != cudaSuccess ||
-      (e = set_crt_attr<10>()) != cudaSuccess || (e = set_crt_attr<11>()) != cudaSuccess ||
-      (e = set_crt_attr<12>()) != cudaSuccess || (e = set_crt_attr<13>()) != cudaSuccess ||
-      (e = set_crt_attr<14>()) != cudaSuccess || (e = set_crt_attr<15>()) != cudaSuccess ||
-      (e = set_crt_attr<16>()) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(k_crt_mixed<2, kCrtMixedSplit>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)) !=
-          cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_crt_mixed<kCrtMixedSplit + 1, kMaxPrimes>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)) !=
-          cudaSuccess)
-    return e;
+  for (auto fn : {k_crt_mixed<2, kCrtMixedSplit, false>, k_crt_mixed<2, kCrtMixedSplit, true>,
+                  k_crt_mixed<kCrtMixedSplit + 1, kMaxPrimes, false>,
+                  k_crt_mixed<kCrtMixedSplit + 1, kMaxPrimes, true>})
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kCrtSmemLimit)) != cudaSuccess)
+      return e;
   for (auto fn : {k_contract_tc<16, 128>, k_contract_tc<8, 128>, k_contract_tc<4, 128>,
                   k_contract_tc<2, 128>, k_contract_tc<1, 128>, k_contract_tc<16, 256>,
                   k_contract_tc<8, 256>, k_contract_tc<4, 256>, k_contract_tc<2, 256>,

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "mpzmm_internal.h"
 
 namespace mpzmm {
@@ -86,23 +88,29 @@ cudaError_t launch_contract_tc(const ProdDesc* prods, const ContractItem* items,
                                uint32_t* res, const int* shapes, int nshapes, int* status,
                                cudaStream_t st, int stall = 0);
 
-// CRT + recompose + sign for `count` output entries with P primes; rmin is
-// the narrowest coefficient width among them (it sizes the shared scratch).
-cudaError_t launch_crt_recompose(const InvDesc* descs, const uint32_t* idx, int count, int P,
-                                 const uint32_t* res, uint32_t* out, int32_t* sizes, int rmin,
-                                 cudaStream_t st);
-
-// The same over several prime counts in one launch: high = false takes the
-// entries with 2..kCrtMixedSplit primes, high = true those with more (each
-// launch's entries in idx, longest first); rmin[P] is the narrowest
-// coefficient width among the entries with P primes (0: none).
+// CRT + recompose + sign.  crt_items takes the output entries idx and leaves
+// in it those that a warp each recomposes whole, longest first; entries so
+// long that one warp each would leave the GPU (of `sms` SMs) idle go to
+// segs, their records numbered from *nrecs (advanced).
+// launch_crt_mixed runs both lists over several prime counts: high = false
+// takes entries with 2..kCrtMixedSplit primes, high = true those with more;
+// rmin[P] is the narrowest coefficient width among the entries with P primes
+// (0: none; it sizes the scratch).  One kernel for the whole entries, two
+// for the segments.
 constexpr int kCrtMixedSplit = 10;
-struct CrtScratch {
-  int cmax[kMaxPrimes + 1];  // tile coefficients per prime count
-  int warp_words;            // scratch words of one warp
-};
-cudaError_t launch_crt_mixed(const InvDesc* descs, const uint32_t* idx, int count, bool high,
-                             const int* rmin, const uint32_t* res, uint32_t* out, int32_t* sizes,
+void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, uint32_t* nrecs,
+               std::vector<CrtItem>* segs);
+constexpr int kCrtSegLaunches = 2;
+cudaError_t launch_crt_mixed(const InvDesc* descs, const CrtItem* segs, int nsegs,
+                             const uint32_t* idx, int count, bool high, const int* rmin,
+                             const uint32_t* res, uint32_t* out, int32_t* sizes, CrtRec* recs,
                              cudaStream_t st);
+// The same over entries 0 .. count - 1 that are all alike (`words` words, P
+// primes, r bits a coefficient), without a list: crt_uniform splits them
+// (into at most max_recs segments in all).
+CrtUniform crt_uniform(uint32_t words, uint32_t count, int sms, uint64_t max_recs);
+cudaError_t launch_crt_uniform(const InvDesc* descs, int count, CrtUniform u, int P, int r,
+                               const uint32_t* res, uint32_t* out, int32_t* sizes, CrtRec* recs,
+                               cudaStream_t st);
 
 }  // namespace mpzmm

@@ -133,4 +133,32 @@ struct CtaItem {
   uint8_t P;
 };
 
+// Work item of one warp of the CRT kernel: words [w0, w1) of output entry
+// `inv` (all of them, or segment `seg` of the entry's `nseg`, whose records
+// start at `rec`).
+struct CrtItem {
+  uint32_t inv;
+  uint32_t w0, w1;
+  uint32_t rec, seg, nseg;
+};
+
+// Entries that are all alike: `words` words each, in nseg segments of `step`
+// words (the last one shorter).
+struct CrtUniform {
+  uint32_t words = 0, nseg = 1, step = 0;
+};
+
+// What k_crt_finish needs of a segment: for each carry c - 1 into it, its
+// first and last nonzero word, its last word that is not all ones and its
+// top bit; the transfer function from the carry in to the carry out; and
+// whether the warp that wrote it did not know the carry in (then it wrote
+// the words for 0).
+struct CrtRec {
+  int32_t first_nz[3], last_nz[3], last_no[3], top[3];
+  uint32_t tf;
+  int32_t open;
+  int32_t pad[2];
+};
+static_assert(sizeof(CrtRec) == 64, "records are counted in residue words");
+
 }  // namespace mpzmm

@@ -53,6 +53,7 @@ struct DeviceState {
   uint8_t* scratch = nullptr;
   uint2* twf = nullptr;
   uint2* twi = nullptr;
+  int sms = 0;
 };
 DeviceState g_dev[kMaxDevices];
 std::mutex g_mu;                                   // serialises the host side
@@ -74,6 +75,8 @@ int setup_device(int dev, DeviceState** out) {
       return cufail(e, "cudaGetSymbolAddress(twiddles)");
     if ((e = cudaGetSymbolAddress((void**)&s.twi, g_noalloc_twi)) != cudaSuccess)
       return cufail(e, "cudaGetSymbolAddress(twiddles)");
+    if ((e = cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+      return cufail(e, "cudaDeviceGetAttribute");
     const Moduli& M = moduli();
     if ((e = upload_constants(M.pc, &M.crt)) != cudaSuccess) return cufail(e, "constants");
     if ((e = init_kernel_attributes()) != cudaSuccess) return cufail(e, "kernel attributes");
@@ -227,6 +230,11 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
     d.entry = (uint32_t)i;
     idx[na + nb + i] = (uint32_t)i;
   }
+  // segments of the results; their records take the place of the operands'
+  // residues, which nothing reads after the contraction
+  const CrtUniform crt =
+      crt_uniform((uint32_t)(2 * prm.out_limbs), (uint32_t)nc, ds->sms,
+                  (uint64_t)(na + nb) * poly / (sizeof(CrtRec) / sizeof(uint32_t)));
   uint8_t* dd = ds->scratch;
   uint32_t* dres = reinterpret_cast<uint32_t*>(ds->scratch + desc_bytes);
   // every check has passed: only now is anything of the caller's touched.
@@ -251,9 +259,9 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
       (e = launch_contract(dpd, ditems, (int)nitems, dres, s)) != cudaSuccess ||
       (e = launch_inv_ntt(dinv, didx + na + nb, (int)nc, P, lgN, dres, ds->twi, s)) !=
           cudaSuccess ||
-      (e = launch_crt_recompose(dinv, didx + na + nb, (int)nc, P, dres,
-                                reinterpret_cast<uint32_t*>(d_c_limbs), d_c_sizes, r, s)) !=
-          cudaSuccess)
+      (e = launch_crt_uniform(dinv, (int)nc, crt, P, r, dres,
+                              reinterpret_cast<uint32_t*>(d_c_limbs), d_c_sizes,
+                              reinterpret_cast<CrtRec*>(dres), s)) != cudaSuccess)
     return cufail(e, "mpzmm_matmul_noalloc launch");
   return kOk;
 }
