@@ -587,7 +587,6 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
   if (built_ || prepared_) return set_error(kErrState, "plan already built");
   check_bounds_ = context().check_bounds;
   prods_ = std::move(prods);
-  const int block_freqs = contract_block_freqs();
   params_.resize(prods_.size());
   zero_prod_.assign(prods_.size(), 0);
 
@@ -595,6 +594,7 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
   std::map<int, Group> recg;
   std::map<int, int64_t> rec_min_r;
 
+  std::vector<uint32_t> cc_prods;  // products contracted on CUDA cores
   uint64_t out_entry = 0;
   const uint64_t* host_end = nullptr;  // end of the previous entry's host limbs
   uintptr_t run_pinned_end = 0;        // end of the pinned range of the current run (0: none)
@@ -762,10 +762,10 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     const uint32_t prod_index = (uint32_t)pd_.size();
     pd_.push_back(pd);
     // tensor-core items cover blocks of at most kTcBlock rows and columns
-    // of C (the launch is sized for the blocks' shapes); CUDA-core items
-    // cover all of C
-    const int rbs = use_tc ? (m + kTcBlock - 1) / kTcBlock : 1;
-    const int cbs = use_tc ? (n + kTcBlock - 1) / kTcBlock : 1;
+    // of C (the launch is sized for the blocks' shapes); CUDA-core items are
+    // cut when every product is known
+    const int rbs = (m + kTcBlock - 1) / kTcBlock;
+    const int cbs = (n + kTcBlock - 1) / kTcBlock;
     if (use_tc)
       for (int rb = 0; rb < rbs; ++rb)
         for (int cb = 0; cb < cbs; ++cb) {
@@ -776,17 +776,17 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
             seen = tc_shapes_[q] == bm && tc_shapes_[q + 1] == k && tc_shapes_[q + 2] == bn;
           if (!seen) tc_shapes_.insert(tc_shapes_.end(), {bm, k, bn});
         }
-    const uint64_t fstep = use_tc ? (uint64_t)kTcFreqsPerCta : (uint64_t)block_freqs;
-    for (int j = 0; j < P; ++j)
-      for (uint64_t h0 = 0; h0 < N; h0 += fstep)
+    if (!use_tc) cc_prods.push_back(prod_index);
+    for (int j = 0; use_tc && j < P; ++j)
+      for (uint64_t h0 = 0; h0 < N; h0 += (uint64_t)kTcFreqsPerCta)
         for (int rb = 0; rb < rbs; ++rb)
           for (int cb = 0; cb < cbs; ++cb) {
-            ContractItem it;
+            TcItem it;
             it.prod = prod_index;
             it.prime = (uint16_t)j;
-            it.pad = (uint16_t)((rb << 8) | cb);  // block of C (tensor cores only)
+            it.pad = (uint16_t)((rb << 8) | cb);  // block of C
             it.h0 = (uint32_t)h0;
-            (use_tc ? tc_items_ : items_).push_back(it);
+            tc_items_.push_back(it);
           }
     const uint64_t ncoef_c = (uint64_t)(prm.lenA + prm.lenB - 1);
     Group& ig = invg[{lgN, P}];
@@ -821,6 +821,7 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     }
   }
   if (out_entry > 0x7fffffffULL) return set_error(kErrTooLarge, "too many output entries");
+  contract_items(pd_.data(), cc_prods, context().num_sms, &items_);
 
   // launch groups and the shared index array
   // Transforms: team-sized classes (lgN >= 3) are merged into one launch per
@@ -928,7 +929,7 @@ int Plan::bind(Workspace* ws) {
   off_pd_ = align16(off_inv_ + inv_.size() * sizeof(InvDesc));
   off_items_ = align16(off_pd_ + pd_.size() * sizeof(ProdDesc));
   off_tc_ = align16(off_items_ + items_.size() * sizeof(ContractItem));
-  off_idx_ = align16(off_tc_ + tc_items_.size() * sizeof(ContractItem));
+  off_idx_ = align16(off_tc_ + tc_items_.size() * sizeof(TcItem));
   off_cta_ = align16(off_idx_ + idx_all_.size() * sizeof(uint32_t));
   off_crt_ = align16(off_cta_ + cta_items_.size() * sizeof(CtaItem));
   desc_bytes_ = align16(off_crt_ + crt_items_.size() * sizeof(CrtItem));
@@ -944,7 +945,7 @@ int Plan::bind(Workspace* ws) {
   if (!items_.empty())
     std::memcpy(hd + off_items_, items_.data(), items_.size() * sizeof(ContractItem));
   if (!tc_items_.empty())
-    std::memcpy(hd + off_tc_, tc_items_.data(), tc_items_.size() * sizeof(ContractItem));
+    std::memcpy(hd + off_tc_, tc_items_.data(), tc_items_.size() * sizeof(TcItem));
   if (!idx_all_.empty())
     std::memcpy(hd + off_idx_, idx_all_.data(), idx_all_.size() * sizeof(uint32_t));
   if (!cta_items_.empty())
@@ -955,7 +956,7 @@ int Plan::bind(Workspace* ws) {
   d_inv_ = reinterpret_cast<InvDesc*>(ws_->d_desc + off_inv_);
   d_pd_ = reinterpret_cast<ProdDesc*>(ws_->d_desc + off_pd_);
   d_items_ = reinterpret_cast<ContractItem*>(ws_->d_desc + off_items_);
-  d_tc_items_ = reinterpret_cast<ContractItem*>(ws_->d_desc + off_tc_);
+  d_tc_items_ = reinterpret_cast<TcItem*>(ws_->d_desc + off_tc_);
   d_idx_ = reinterpret_cast<uint32_t*>(ws_->d_desc + off_idx_);
   d_cta_ = reinterpret_cast<CtaItem*>(ws_->d_desc + off_cta_);
   d_crt_ = reinterpret_cast<CrtItem*>(ws_->d_desc + off_crt_);

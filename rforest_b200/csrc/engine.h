@@ -331,7 +331,7 @@ class Plan {
   std::vector<InvDesc> inv_;
   std::vector<ProdDesc> pd_;
   std::vector<ContractItem> items_;     // CUDA-core contraction work
-  std::vector<ContractItem> tc_items_;  // tensor-core contraction work
+  std::vector<TcItem> tc_items_;        // tensor-core contraction work
   std::vector<int> tc_shapes_;  // distinct (m, k, n) of the tensor-core products
   std::vector<Group> fwd_groups_, inv_groups_, rec_groups_;
   std::vector<uint32_t> idx_all_;
@@ -388,7 +388,7 @@ class Plan {
   InvDesc* d_inv_ = nullptr;
   ProdDesc* d_pd_ = nullptr;
   ContractItem* d_items_ = nullptr;
-  ContractItem* d_tc_items_ = nullptr;
+  TcItem* d_tc_items_ = nullptr;
   size_t off_tc_ = 0;
   uint32_t* d_idx_ = nullptr;
   bool built_ = false;

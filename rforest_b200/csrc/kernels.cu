@@ -159,146 +159,173 @@ __global__ void k_inv_ntt(const InvDesc* __restrict__ descs,
   const uint32_t p = c_primes[j].p;
   const int N = 1 << d.lgN;
   uint32_t* io = res + d.res_off + (uint64_t)j * (uint64_t)N;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) sm[i] = io[i];
+  // the contraction leaves values in [0, 2p); these butterflies want [0, p)
+  for (int i = threadIdx.x; i < N; i += blockDim.x) sm[i] = min(io[i], io[i] - p);
   __syncthreads();
   ntt_inv_smem(sm, d.lgN, twi + (size_t)j * kTwStride, p);
   for (int i = threadIdx.x; i < N; i += blockDim.x) io[i] = sm[i];
 }
 
 // ---------------------------------------------------------------------------
-// Contraction on CUDA cores.  One thread per frequency h; it walks the m x n
-// outputs in register tiles of TI x TJ (2 or 4 each, chosen per product and
-// stored in ProdDesc::pad), loading TI + TJ residues per TI * TJ products.
+// Contraction on CUDA cores.  One thread per residue position x of a
+// polynomial (prime x >> lgN, frequency x mod N: the primes' residues follow
+// one another, so a block takes 128 positions whatever the transform's
+// length); it walks its share of the m x n outputs in register tiles of
+// TI x TJ (1 to 4 each, chosen per product and stored in ProdDesc::pad),
+// loading TI + TJ residues per TI * TJ products.
 // Edge tiles clamp their row/column to the last one (in-bounds duplicate
-// work, results discarded).  Products of residues < p < 2^30 are < 2^60, so
-// sixteen of them accumulate exactly in 64 bits before a Montgomery fold (the
+// work, results discarded).  Products of residues < p < 2^30 are at most
+// 2^60 - 2^31, so sixteen of them accumulate exactly in 64 bits (the
 // reference reduces every 16 terms for the same reason with 128-bit
-// accumulators, src/lib/mpnfft.c:621-627).  Outputs carry a factor 2^-32
-// that the CRT stage removes.
+// accumulators, src/lib/mpnfft.c:621-627); then the high word is folded down
+// and twelve more fit.  Outputs carry a factor 2^-32 that the CRT stage
+// removes.
+// The tiles of a block of positions are split over several CTAs where whole
+// ones would not fill the GPU: a 2000 x 1 by 1 x 1 product of 10^4-bit
+// integers (1408 positions) took 295 us in 11 CTAs, 16 split.
+// Bound by its loads (operands straight from L2, DRAM at about 40 % of its
+// rate): up to four terms' loads go out together, and 80 registers leave
+// six CTAs an SM.  1314 us for the first 512 products of the default batch,
+// 1400 before the terms past a multiple of four were loaded together and
+// the folds cut to one multiply-add; 1360 at 128 registers, 1470 at 64.
+// Staging a block's operands in shared memory (cp.async, two buffers)
+// measured 1850: too little work a CTA for its two waits.
 // ---------------------------------------------------------------------------
 constexpr int kContractThreads = 128;
 
-// x mod p for any 64-bit x (Barrett on the high word, then REDC of the
-// reduced value times 2^32): keeps the accumulator's value, not its
-// Montgomery image, so folds can be repeated.
-__device__ __forceinline__ uint64_t fold64(uint64_t x, uint32_t p, uint32_t pinv, uint32_t mu,
-                                           uint32_t r2) {
-  // x = hi 2^32 + lo;  x mod p = REDC((x 2^-32 mod p) * 2^64 mod p)
-  const uint32_t t = redc64(x, p, pinv, mu);           // x 2^-32 mod p
-  return redc((uint64_t)t * r2, p, pinv);              // x mod p
+constexpr int kContractFirst = 16;  // products a fresh accumulator holds
+constexpr int kContractMore = 12;   // further ones after a fold
+
+// The high word folded down: lo + hi (2^32 mod p), below 2^62 + 2^32.
+__device__ __forceinline__ uint64_t fold64(uint64_t x, uint32_t b32) {
+  return (uint64_t)(uint32_t)(x >> 32) * b32 + (uint32_t)x;
+}
+
+// R terms (1 to 4) of a tile, their loads issued together.
+template <int TI, int TJ, int R>
+__device__ __forceinline__ void contract_terms(uint64_t (&acc)[TI][TJ],
+                                               const uint32_t* __restrict__ A,
+                                               const uint32_t* __restrict__ B,
+                                               const uint32_t (&ao)[TI], const uint32_t (&bo)[TJ],
+                                               uint32_t stride, uint32_t bstep, uint32_t b32,
+                                               int& room) {
+  uint32_t av[R][TI], bv[R][TJ];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+#pragma unroll
+    for (int x = 0; x < TI; ++x) av[u][x] = __ldg(A + ao[x] + (uint32_t)u * stride);
+#pragma unroll
+    for (int y = 0; y < TJ; ++y) bv[u][y] = __ldg(B + bo[y] + (uint32_t)u * bstep);
+  }
+  if (room < R) {
+#pragma unroll
+    for (int x = 0; x < TI; ++x)
+#pragma unroll
+      for (int y = 0; y < TJ; ++y) acc[x][y] = fold64(acc[x][y], b32);
+    room = kContractMore;
+  }
+  room -= R;
+#pragma unroll
+  for (int u = 0; u < R; ++u)
+#pragma unroll
+    for (int x = 0; x < TI; ++x)
+#pragma unroll
+      for (int y = 0; y < TJ; ++y) acc[x][y] += (uint64_t)av[u][x] * bv[u][y];
 }
 
 template <int TI, int TJ>
-__device__ __forceinline__ void contract_tiles(const ProdDesc& d, int j, uint32_t h,
-                                               uint32_t* __restrict__ res) {
-  const int N = 1 << d.lgN;
+__device__ __forceinline__ void contract_tiles(const ProdDesc& d, const ContractItem& it,
+                                               uint32_t pos, uint32_t* __restrict__ res) {
+  const int j = (int)(pos >> d.lgN);
   const uint32_t p = c_primes[j].p;
   const uint32_t pinv = c_primes[j].pinv;
-  const uint32_t mu = c_primes[j].mu;
-  const uint32_t r2 = c_primes[j].r2;
-  const uint32_t stride = (uint32_t)d.P * (uint32_t)N;  // words between polynomials
-  const uint64_t base = (uint64_t)j * (uint64_t)N + h;
-  const uint32_t* __restrict__ A = res + d.a_res + base;
-  const uint32_t* __restrict__ B = res + d.b_res + base;
-  uint32_t* C = res + d.c_res + base;
+  const uint32_t b32 = c_primes[j].b32;
+  const uint32_t stride = (uint32_t)d.P << d.lgN;  // words between polynomials
+  const uint32_t* __restrict__ A = res + d.a_res + pos;
+  const uint32_t* __restrict__ B = res + d.b_res + pos;
+  uint32_t* C = res + d.c_res + pos;
   const int m = d.m, k = d.k, n = d.n;
   const uint32_t bstep = (uint32_t)n * stride;
-  for (int i0 = 0; i0 < m; i0 += TI) {
-    for (int l0 = 0; l0 < n; l0 += TJ) {
-      uint32_t ao[TI], bo[TJ];  // word offsets of the tile's rows / columns
+  const uint32_t tn = (uint32_t)(n + TJ - 1) / TJ;  // tiles of a row of them
+  int i0 = (int)(it.t0 / tn) * TI, l0 = (int)(it.t0 % tn) * TJ;
+  for (uint32_t t = 0; t < it.nt; ++t) {
+    uint32_t ao[TI], bo[TJ];  // word offsets of the tile's rows / columns
 #pragma unroll
-      for (int x = 0; x < TI; ++x) {
-        const int ii = (i0 + x) < m ? (i0 + x) : (m - 1);
-        ao[x] = (uint32_t)ii * (uint32_t)k * stride;
-      }
+    for (int x = 0; x < TI; ++x) {
+      const int ii = (i0 + x) < m ? (i0 + x) : (m - 1);
+      ao[x] = (uint32_t)ii * (uint32_t)k * stride;
+    }
+#pragma unroll
+    for (int y = 0; y < TJ; ++y) {
+      const int ll = (l0 + y) < n ? (l0 + y) : (n - 1);
+      bo[y] = (uint32_t)ll * stride;
+    }
+    uint64_t acc[TI][TJ];
+#pragma unroll
+    for (int x = 0; x < TI; ++x)
+#pragma unroll
+      for (int y = 0; y < TJ; ++y) acc[x][y] = 0;
+    int room = kContractFirst;
+    const uint32_t* __restrict__ Aq = A;
+    const uint32_t* __restrict__ Bq = B;
+    for (int q = k; q >= 4; q -= 4) {
+      contract_terms<TI, TJ, 4>(acc, Aq, Bq, ao, bo, stride, bstep, b32, room);
+      Aq += 4 * (uint64_t)stride;
+      Bq += 4 * (uint64_t)bstep;
+    }
+    switch (k & 3) {
+      case 3: contract_terms<TI, TJ, 3>(acc, Aq, Bq, ao, bo, stride, bstep, b32, room); break;
+      case 2: contract_terms<TI, TJ, 2>(acc, Aq, Bq, ao, bo, stride, bstep, b32, room); break;
+      case 1: contract_terms<TI, TJ, 1>(acc, Aq, Bq, ao, bo, stride, bstep, b32, room); break;
+    }
+#pragma unroll
+    for (int x = 0; x < TI; ++x) {
+      if (i0 + x >= m) continue;
 #pragma unroll
       for (int y = 0; y < TJ; ++y) {
-        const int ll = (l0 + y) < n ? (l0 + y) : (n - 1);
-        bo[y] = (uint32_t)ll * stride;
+        if (l0 + y >= n) continue;
+        // the value times 2^-32 (the Montgomery factor the CRT removes), in
+        // [0, 2p): the fold leaves T < 2^62 + 2^32, its REDC is at most
+        // p + 2^30 + 1, and p is above 2^29
+        const uint64_t T = fold64(acc[x][y], b32);
+        const uint32_t v = (uint32_t)((T + (uint64_t)((uint32_t)T * pinv) * p) >> 32);
+        C[(uint32_t)((i0 + x) * n + (l0 + y)) * stride] = min(v, v - p);
       }
-      uint64_t acc[TI][TJ];
-#pragma unroll
-      for (int x = 0; x < TI; ++x)
-#pragma unroll
-        for (int y = 0; y < TJ; ++y) acc[x][y] = 0;
-      // acc < p + 15 p^2 < 2^64 between folds
-      int since = 0;
-      int q = 0;
-      for (; q + 4 <= k; q += 4) {
-        uint32_t av[4][TI], bv[4][TJ];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-          for (int x = 0; x < TI; ++x) av[u][x] = __ldg(A + ao[x] + (uint32_t)(q + u) * stride);
-#pragma unroll
-          for (int y = 0; y < TJ; ++y) bv[u][y] = __ldg(B + bo[y] + (uint32_t)(q + u) * bstep);
-        }
-        if (since + 4 > 15) {
-#pragma unroll
-          for (int x = 0; x < TI; ++x)
-#pragma unroll
-            for (int y = 0; y < TJ; ++y) acc[x][y] = fold64(acc[x][y], p, pinv, mu, r2);
-          since = 0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int x = 0; x < TI; ++x)
-#pragma unroll
-            for (int y = 0; y < TJ; ++y) acc[x][y] += (uint64_t)av[u][x] * bv[u][y];
-        since += 4;
-      }
-      for (; q < k; ++q) {
-        if (since + 1 > 15) {
-#pragma unroll
-          for (int x = 0; x < TI; ++x)
-#pragma unroll
-            for (int y = 0; y < TJ; ++y) acc[x][y] = fold64(acc[x][y], p, pinv, mu, r2);
-          since = 0;
-        }
-        uint32_t av[TI], bv[TJ];
-#pragma unroll
-        for (int x = 0; x < TI; ++x) av[x] = __ldg(A + ao[x] + (uint32_t)q * stride);
-#pragma unroll
-        for (int y = 0; y < TJ; ++y) bv[y] = __ldg(B + bo[y] + (uint32_t)q * bstep);
-#pragma unroll
-        for (int x = 0; x < TI; ++x)
-#pragma unroll
-          for (int y = 0; y < TJ; ++y) acc[x][y] += (uint64_t)av[x] * bv[y];
-        ++since;
-      }
-#pragma unroll
-      for (int x = 0; x < TI; ++x) {
-        if (i0 + x >= m) continue;
-#pragma unroll
-        for (int y = 0; y < TJ; ++y) {
-          if (l0 + y >= n) continue;
-          // the value times 2^-32 (the Montgomery factor the CRT removes)
-          C[(uint32_t)((i0 + x) * n + (l0 + y)) * stride] = redc64(acc[x][y], p, pinv, mu);
-        }
-      }
+    }
+    l0 += TJ;
+    if (l0 >= n) {
+      l0 = 0;
+      i0 += TI;
     }
   }
 }
 
-__global__ void __launch_bounds__(kContractThreads)
+// items == nullptr: product 0 alone, its blocks of positions and groups of
+// u.per tiles in grid order
+__global__ void __launch_bounds__(kContractThreads, 6)
 k_contract(const ProdDesc* __restrict__ prods, const ContractItem* __restrict__ items,
-           uint32_t* __restrict__ res) {
-  const ContractItem it = items[blockIdx.x];
+           ContractUniform u, uint32_t* __restrict__ res) {
+  ContractItem it;
+  if (items) {
+    it = items[blockIdx.x];
+  } else {
+    const uint32_t g = blockIdx.x / u.blocks;
+    it.prod = 0;
+    it.x0 = (blockIdx.x - g * u.blocks) * (uint32_t)kContractThreads;
+    it.t0 = g * u.per;
+    it.nt = min(u.per, u.tiles - it.t0);
+  }
   const ProdDesc d = prods[it.prod];
-  const int N = 1 << d.lgN;
-  const uint32_t h = it.h0 + threadIdx.x;
-  if (h >= (uint32_t)N) return;
-  switch (d.pad) {  // tile shape 3 (TI - 2) + (TJ - 2), uniform over the CTA
-    case 8: contract_tiles<4, 4>(d, it.prime, h, res); break;
-    case 7: contract_tiles<4, 3>(d, it.prime, h, res); break;
-    case 6: contract_tiles<4, 2>(d, it.prime, h, res); break;
-    case 5: contract_tiles<3, 4>(d, it.prime, h, res); break;
-    case 4: contract_tiles<3, 3>(d, it.prime, h, res); break;
-    case 3: contract_tiles<3, 2>(d, it.prime, h, res); break;
-    case 2: contract_tiles<2, 4>(d, it.prime, h, res); break;
-    case 1: contract_tiles<2, 3>(d, it.prime, h, res); break;
-    default: contract_tiles<2, 2>(d, it.prime, h, res); break;
+  const uint32_t pos = it.x0 + threadIdx.x;
+  if (pos >= ((uint32_t)d.P << d.lgN)) return;
+  switch (d.pad) {  // tile shape 4 (TI - 1) + (TJ - 1), uniform over the CTA
+#define MPZMM_TILE(TI, TJ) \
+  case 4 * (TI - 1) + (TJ - 1): contract_tiles<TI, TJ>(d, it, pos, res); break;
+    MPZMM_TILE(4, 4) MPZMM_TILE(4, 3) MPZMM_TILE(4, 2) MPZMM_TILE(4, 1)
+    MPZMM_TILE(3, 4) MPZMM_TILE(3, 3) MPZMM_TILE(3, 2) MPZMM_TILE(3, 1)
+    MPZMM_TILE(2, 4) MPZMM_TILE(2, 3) MPZMM_TILE(2, 2) MPZMM_TILE(2, 1)
+    MPZMM_TILE(1, 4) MPZMM_TILE(1, 3) MPZMM_TILE(1, 2) MPZMM_TILE(1, 1)
+#undef MPZMM_TILE
   }
 }
 
@@ -1568,7 +1595,7 @@ __device__ __forceinline__ void load_freqs(const uint32_t* __restrict__ blk, uin
 // quadrant), 256 where two do, 512 where one CTA has it to itself.
 template <int F, int NT>
 __global__ void __launch_bounds__(NT, 512 / NT)
-k_contract_tc(const ProdDesc* __restrict__ prods, const ContractItem* __restrict__ items,
+k_contract_tc(const ProdDesc* __restrict__ prods, const TcItem* __restrict__ items,
               uint32_t* __restrict__ res, int bufcols, int* __restrict__ status, int stall) {
   extern __shared__ __align__(1024) uint8_t tsm[];
   __shared__ __align__(8) uint64_t bars[2];
@@ -1576,7 +1603,7 @@ k_contract_tc(const ProdDesc* __restrict__ prods, const ContractItem* __restrict
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const ContractItem it = items[blockIdx.x];
+  const TcItem it = items[blockIdx.x];
   const ProdDesc d = prods[it.prod];
   // the item's block of C: rows i_base .. + m, columns l_base .. + n (at
   // most kBlock each); m, n below are the block's, d.m, d.n the product's
@@ -2191,11 +2218,54 @@ cudaError_t launch_inv_ntt(const InvDesc* descs, const uint32_t* idx, int count,
 cudaError_t launch_contract(const ProdDesc* prods, const ContractItem* items, int count,
                             uint32_t* res, cudaStream_t st) {
   if (count == 0) return cudaSuccess;
-  k_contract<<<count, kContractThreads, 0, st>>>(prods, items, res);
+  k_contract<<<count, kContractThreads, 0, st>>>(prods, items, ContractUniform{}, res);
   return cudaGetLastError();
 }
 
-int contract_block_freqs() { return kContractThreads; }
+// Tiles of product d, and the blocks of positions of its polynomials.
+static uint32_t contract_tiles_of(const ProdDesc& d) {
+  const uint32_t ti = d.pad / 4 + 1u, tj = d.pad % 4 + 1u;
+  return ((d.m + ti - 1) / ti) * ((d.n + tj - 1) / tj);
+}
+static uint32_t contract_blocks_of(const ProdDesc& d) {
+  return (((uint32_t)d.P << d.lgN) + kContractThreads - 1) / kContractThreads;
+}
+
+// Tiles a CTA takes where a launch has `work` tiles (over all blocks of
+// positions): one while the launch is below four times the CTAs that run
+// at once (six an SM), more as it grows.
+static uint32_t contract_per(uint64_t work, int sms) {
+  const uint64_t per = work / ((uint64_t)(sms > 0 ? sms : 1) * 24);
+  return per < 1 ? 1u : (uint32_t)std::min<uint64_t>(per, 0xffffffffu);
+}
+
+void contract_items(const ProdDesc* prods, const std::vector<uint32_t>& which, int sms,
+                    std::vector<ContractItem>* items) {
+  uint64_t work = 0;
+  for (const uint32_t q : which)
+    work += (uint64_t)contract_tiles_of(prods[q]) * contract_blocks_of(prods[q]);
+  const uint32_t per = contract_per(work, sms);
+  for (const uint32_t q : which) {
+    const uint32_t tiles = contract_tiles_of(prods[q]), nb = contract_blocks_of(prods[q]);
+    // equal groups: no short one at the end
+    const uint32_t groups = (tiles + per - 1) / per, each = (tiles + groups - 1) / groups;
+    for (uint32_t b = 0; b < nb; ++b)
+      for (uint32_t t = 0; t < tiles; t += each)
+        items->push_back(ContractItem{q, b * (uint32_t)kContractThreads, t,
+                                      std::min(each, tiles - t)});
+  }
+}
+
+cudaError_t launch_contract_one(const ProdDesc* prod, const ProdDesc& d, int sms, uint32_t* res,
+                                cudaStream_t st) {
+  ContractUniform u;
+  u.blocks = contract_blocks_of(d);
+  u.tiles = contract_tiles_of(d);
+  u.per = std::min(u.tiles, contract_per((uint64_t)u.tiles * u.blocks, sms));
+  const uint32_t groups = (u.tiles + u.per - 1) / u.per;
+  k_contract<<<groups * u.blocks, kContractThreads, 0, st>>>(prod, nullptr, u, res);
+  return cudaGetLastError();
+}
 
 __device__ __forceinline__ bool fwd_in_bounds(const FwdDesc& f, const BoundsCaps& c) {
   if (f.lgN > kMaxLgN || f.P > kMaxPrimes) return false;
@@ -2309,7 +2379,7 @@ static bool tc_launch_config(const int* shapes, int nshapes, int* bufcols, int* 
 
 template <int F>
 static void launch_tc_f(int count, int smem, int threads, cudaStream_t st,
-                        const ProdDesc* prods, const ContractItem* items, uint32_t* res,
+                        const ProdDesc* prods, const TcItem* items, uint32_t* res,
                         int bufcols, int* status, int stall) {
   if (threads == 512)
     k_contract_tc<F, 512><<<count, 512, smem, st>>>(prods, items, res, bufcols, status, stall);
@@ -2319,7 +2389,7 @@ static void launch_tc_f(int count, int smem, int threads, cudaStream_t st,
     k_contract_tc<F, 128><<<count, 128, smem, st>>>(prods, items, res, bufcols, status, stall);
 }
 
-cudaError_t launch_contract_tc(const ProdDesc* prods, const ContractItem* items, int count,
+cudaError_t launch_contract_tc(const ProdDesc* prods, const TcItem* items, int count,
                                uint32_t* res, const int* shapes, int nshapes, int* status,
                                cudaStream_t st, int stall) {
   if (count == 0) return cudaSuccess;

@@ -52,7 +52,12 @@ constexpr int kLargeLaunches = 2;  // kernel launches per direction of a four-st
 // CUDA-core contraction over `count` work items.
 cudaError_t launch_contract(const ProdDesc* prods, const ContractItem* items, int count,
                             uint32_t* res, cudaStream_t st);
-int contract_block_freqs();
+// The work of the products `which` (indices into prods), appended to items.
+void contract_items(const ProdDesc* prods, const std::vector<uint32_t>& which, int sms,
+                    std::vector<ContractItem>* items);
+// One product alone (its descriptor on the device and here), without a list.
+cudaError_t launch_contract_one(const ProdDesc* prod, const ProdDesc& d, int sms, uint32_t* res,
+                                cudaStream_t st);
 // writes the device-held signed sizes (and coefficient counts) of `count`
 // forward descriptors
 cudaError_t launch_fix_sizes(FwdDesc* descs, int count, const int32_t* sizes, cudaStream_t st);
@@ -84,7 +89,7 @@ cudaError_t launch_check_bounds(const FwdDesc* fwd, int nfwd, const InvDesc* inv
 bool contract_tc_eligible(int m, int k, int n);
 int contract_tc_freqs();
 int tc_smem_bytes(int m, int k, int n, int F);
-cudaError_t launch_contract_tc(const ProdDesc* prods, const ContractItem* items, int count,
+cudaError_t launch_contract_tc(const ProdDesc* prods, const TcItem* items, int count,
                                uint32_t* res, const int* shapes, int nshapes, int* status,
                                cudaStream_t st, int stall = 0);
 

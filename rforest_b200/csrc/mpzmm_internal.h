@@ -112,14 +112,28 @@ struct ProdDesc {
   uint16_t m, k, n;
   uint16_t lgN;
   uint16_t P;
-  uint16_t pad;        // contraction register tile TI x TJ (2..4 each): 3 (TI - 2) + TJ - 2
+  uint16_t pad;        // contraction register tile TI x TJ (1..4 each): 4 (TI - 1) + TJ - 1
 };
 
-// Work item of the contraction: one product, one prime, one frequency block.
+// Work item of the CUDA-core contraction: register tiles t0 .. t0 + nt - 1 (row
+// by row) of one product, at the 128 residue positions from x0.
 struct ContractItem {
   uint32_t prod;
+  uint32_t x0;
+  uint32_t t0, nt;
+};
+
+// The work of one product alone: blocks of positions, tiles, tiles a CTA.
+struct ContractUniform {
+  uint32_t blocks = 0, tiles = 0, per = 0;
+};
+
+// Work item of the tensor-core contraction: one product, one prime, one
+// block of frequencies, one block of C.
+struct TcItem {
+  uint32_t prod;
   uint16_t prime;
-  uint16_t pad;        // tensor cores: block of C, (row block << 8) | column block
+  uint16_t pad;        // block of C, (row block << 8) | column block
   uint32_t h0;         // first frequency of the block
 };
 

@@ -159,19 +159,19 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
 
   const int P = prm.P, lgN = prm.lgN, r = prm.r;
   const uint64_t N = (uint64_t)1 << lgN, poly = (uint64_t)P * N;
-  const int bf = contract_block_freqs();
-  const int64_t nitems = (int64_t)P * (int64_t)((N + bf - 1) / bf);
-  // descriptor blob: fwd (A then B), inv, prod, items, index lists
+  // descriptor blob: fwd (A then B), inv, prod, index lists; the limits
+  // below count 12 bytes for each 128 frequencies of a prime besides
   const size_t off_fwd = 0;
   const size_t off_inv = align256(off_fwd + sizeof(FwdDesc) * (size_t)(na + nb));
   const size_t off_pd = align256(off_inv + sizeof(InvDesc) * (size_t)nc);
-  const size_t off_items = align256(off_pd + sizeof(ProdDesc));
-  const size_t off_idx = align256(off_items + sizeof(ContractItem) * (size_t)nitems);
+  const size_t off_idx = align256(off_pd + sizeof(ProdDesc));
   const size_t desc_bytes = align256(off_idx + sizeof(uint32_t) * (size_t)(na + nb + nc));
+  const size_t counted = align256(off_idx + 12 * (size_t)P * (size_t)((N + 127) / 128)) - off_idx +
+                         desc_bytes;
   const size_t res_bytes = sizeof(uint32_t) * (size_t)(na + nb + nc) * poly;
-  if (desc_bytes > kNoAllocDescBytes || desc_bytes + res_bytes > kNoAllocScratchBytes)
+  if (counted > kNoAllocDescBytes || counted + res_bytes > kNoAllocScratchBytes)
     return set_error(kErrTooLarge,
-                     "mpzmm_matmul_noalloc: needs " + std::to_string(desc_bytes + res_bytes) +
+                     "mpzmm_matmul_noalloc: needs " + std::to_string(counted + res_bytes) +
                          " scratch bytes, the static scratch holds " +
                          std::to_string(kNoAllocScratchBytes));
 
@@ -179,7 +179,6 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
   FwdDesc* fwd = reinterpret_cast<FwdDesc*>(hd + off_fwd);
   InvDesc* inv = reinterpret_cast<InvDesc*>(hd + off_inv);
   ProdDesc* pd = reinterpret_cast<ProdDesc*>(hd + off_pd);
-  ContractItem* items = reinterpret_cast<ContractItem*>(hd + off_items);
   uint32_t* idx = reinterpret_cast<uint32_t*>(hd + off_idx);
   pd->m = (uint16_t)m;
   pd->k = (uint16_t)k;
@@ -208,15 +207,6 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
     f.tile_e = 0;
     idx[i] = (uint32_t)i;
   }
-  int64_t it = 0;
-  for (int j = 0; j < P; ++j)
-    for (uint64_t h0 = 0; h0 < N; h0 += (uint64_t)bf) {
-      items[it].prod = 0;
-      items[it].prime = (uint16_t)j;
-      items[it].pad = 0;
-      items[it].h0 = (uint32_t)h0;
-      ++it;
-    }
   const uint64_t ncoef_c = (uint64_t)(prm.lenA + prm.lenB - 1);
   for (int64_t i = 0; i < nc; ++i) {
     InvDesc& d = inv[i];
@@ -249,14 +239,13 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
   const FwdDesc* dfwd = reinterpret_cast<const FwdDesc*>(dd + off_fwd);
   const InvDesc* dinv = reinterpret_cast<const InvDesc*>(dd + off_inv);
   const ProdDesc* dpd = reinterpret_cast<const ProdDesc*>(dd + off_pd);
-  const ContractItem* ditems = reinterpret_cast<const ContractItem*>(dd + off_items);
   const uint32_t* didx = reinterpret_cast<const uint32_t*>(dd + off_idx);
 
   if ((e = launch_split_fwd(dfwd, didx, (int)na, P, lgN, d_a_limbs, dres, ds->twf, s)) !=
           cudaSuccess ||
       (e = launch_split_fwd(dfwd, didx + na, (int)nb, P, lgN, d_b_limbs, dres, ds->twf, s)) !=
           cudaSuccess ||
-      (e = launch_contract(dpd, ditems, (int)nitems, dres, s)) != cudaSuccess ||
+      (e = launch_contract_one(dpd, *pd, ds->sms, dres, s)) != cudaSuccess ||
       (e = launch_inv_ntt(dinv, didx + na + nb, (int)nc, P, lgN, dres, ds->twi, s)) !=
           cudaSuccess ||
       (e = launch_crt_uniform(dinv, (int)nc, crt, P, r, dres,

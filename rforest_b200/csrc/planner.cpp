@@ -247,8 +247,8 @@ int64_t output_limbs(int k, int64_t a_bits, int64_t b_bits) {
   return (a_bits + b_bits + ceil_log2((uint64_t)k) + 1 + 63) / 64;
 }
 
-// Register tile of the CUDA-core contraction, TI x TJ with 2 <= TI, TJ <= 4,
-// as 3 (TI - 2) + (TJ - 2): the one with the fewest modelled instructions a
+// Register tile of the CUDA-core contraction, TI x TJ with 1 <= TI, TJ <= 4,
+// as 4 (TI - 1) + (TJ - 1): the one with the fewest modelled instructions a
 // frequency and term, tiles x (2 per multiply-add + 3 per load), so a
 // 5 x 5 product takes 3 x 3 tiles (no row or column computed twice over)
 // and a 16 x 16 one 4 x 4 (fewer loads a multiply-add).  On the default
@@ -256,14 +256,15 @@ int64_t output_limbs(int k, int64_t a_bits, int64_t b_bits) {
 // measured 9.77 against 9.87 ms: the contraction waits on its loads more
 // than it issues.
 int contract_tile(int m, int n) {
-  int best = 0, best_cost = -1;
-  for (int ti = 2; ti <= 4; ++ti)
-    for (int tj = 2; tj <= 4; ++tj) {
-      const int tiles = ((m + ti - 1) / ti) * ((n + tj - 1) / tj);
-      const int cost = tiles * (2 * ti * tj + 3 * (ti + tj));
+  int best = 0;
+  int64_t best_cost = -1;
+  for (int ti = 1; ti <= 4; ++ti)
+    for (int tj = 1; tj <= 4; ++tj) {
+      const int64_t tiles = (int64_t)((m + ti - 1) / ti) * ((n + tj - 1) / tj);
+      const int64_t cost = tiles * (2 * ti * tj + 3 * (ti + tj));
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
-        best = 3 * (ti - 2) + (tj - 2);
+        best = 4 * (ti - 1) + (tj - 1);
       }
     }
   return best;
