@@ -831,6 +831,12 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
   auto batch_classes = [&](std::map<std::pair<int, int>, Group>& classes, bool fwd,
                            std::vector<Group>& out) {
     std::map<std::pair<int, int>, Group> var;  // (0 = team, else lgN; D)
+    // CTAs of the stage with all primes each: few are cut by primes
+    uint64_t ctas = 0;
+    for (const auto& kv : classes) {
+      const int64_t G = std::max<int64_t>(1, fwd_team_points() >> kv.second.lgN);
+      ctas += (kv.second.idx.size() + G - 1) / G;
+    }
     for (auto& kv : classes) {
       Group& g = kv.second;
       const int D = fwd ? (g.max_r + 29) / 30 : 0;
@@ -855,15 +861,20 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
       v.D = D;
       if (g.lgN > v.max_lgN) v.max_lgN = g.lgN;
       const size_t G = team ? (size_t)(fwd_team_points() >> g.lgN) : 1;
+      const int chunks = prime_chunks(ctas, g.P, context().num_sms);
+      v.P = std::max(v.P, (g.P + chunks - 1) / chunks);  // most primes a CTA
       for (size_t i = 0; i < g.idx.size(); i += G) {
         const size_t cnt = (g.idx.size() - i) < G ? (g.idx.size() - i) : G;
-        CtaItem it;
+        CtaItem it{};
         it.first = (uint32_t)idx_all_.size();
         it.count = (uint16_t)cnt;
         it.lgN = (uint8_t)g.lgN;
-        it.P = (uint8_t)g.P;
         idx_all_.insert(idx_all_.end(), g.idx.begin() + i, g.idx.begin() + i + cnt);
-        v.items.push_back(it);
+        for (int c = 0; c < chunks; ++c) {
+          it.j0 = (uint8_t)(g.P * c / chunks);
+          it.j1 = (uint8_t)(g.P * (c + 1) / chunks);
+          v.items.push_back(it);
+        }
       }
     }
     for (auto& kv : var) {
@@ -1216,12 +1227,12 @@ int Plan::launch_all(cudaStream_t st, bool timed) {
   int r = fan_out(ws_, st, (int)fwd_run.size(), [&](int i, cudaStream_t s) -> int {
     const Group& g = *fwd_run[i];
     if (g.large)
-      CU(launch_large_fwd(d_fwd_, d_idx_ + g.idx_off, (int)g.idx.size(), g.lgN, g.D,
-                          ws_->d_limbs, ws_->d_res, ctx.d_twf, ctx.twist_f, s),
+      CU(launch_large_fwd(d_fwd_, d_idx_ + g.idx_off, (int)g.idx.size(), g.lgN, g.P, g.D,
+                          ctx.num_sms, ws_->d_limbs, ws_->d_res, ctx.d_twf, ctx.twist_f, s),
          "split+forward NTT launch (four-step)");
     else if (g.batched)
       CU(launch_fwd_items(d_fwd_, d_idx_, d_cta_ + g.item_off, (int)g.items.size(), g.D, g.team,
-                          g.max_lgN, ws_->d_limbs, ws_->d_res, ctx.d_twf, s, g.tiled),
+                          g.max_lgN, g.P, ws_->d_limbs, ws_->d_res, ctx.d_twf, s),
          "split+forward NTT launch");
     else
       CU(launch_split_fwd(d_fwd_, d_idx_ + g.idx_off, (int)g.idx.size(), g.P, g.lgN,
@@ -1242,8 +1253,8 @@ int Plan::launch_all(cudaStream_t st, bool timed) {
   r = fan_out(ws_, st, (int)inv_groups_.size(), [&](int i, cudaStream_t s) -> int {
     const Group& g = inv_groups_[i];
     if (g.large)
-      CU(launch_large_inv(d_inv_, d_idx_ + g.idx_off, (int)g.idx.size(), g.lgN, ws_->d_res,
-                          ctx.d_twi, ctx.twist_i, s),
+      CU(launch_large_inv(d_inv_, d_idx_ + g.idx_off, (int)g.idx.size(), g.lgN, g.P, ctx.num_sms,
+                          ws_->d_res, ctx.d_twi, ctx.twist_i, s),
          "inverse NTT launch (four-step)");
     else if (g.batched)
       CU(launch_inv_items(d_inv_, d_idx_, d_cta_ + g.item_off, (int)g.items.size(), g.team,

@@ -1,6 +1,7 @@
 // sm_100a kernels of the exact matrix-product pipeline.
 //
-//   k_fwd2           limbs -> r-bit coefficients -> 30-bit digits ->
+//   k_fwd_team, k_fwd_cta
+//                    limbs -> r-bit coefficients -> 30-bit digits ->
 //                    residues mod p -> forward NTT, register-blocked passes
 //                    (several small transforms or one large one per CTA)
 //   k_split_fwd      the same, radix 2, one CTA per (entry, prime): tiny
@@ -9,7 +10,8 @@
 //                    CUDA cores (64-bit lazy accumulation, Montgomery fold)
 //   k_contract_tc    the same on tensor cores (tcgen05 kind::i8, exact
 //                    byte split; contract_tc.cuh)
-//   k_inv2           inverse NTT, register-blocked; k_inv_ntt radix 2
+//   k_inv_team, k_inv_cta
+//                    inverse NTT, register-blocked; k_inv_ntt radix 2
 //   k_crt_mixed      explicit CRT to signed multi-word coefficients, then
 //                    sum_i c_i 2^(i r) with carries resolved by a
 //                    carry-lookahead prefix scan over 32-bit output words,
@@ -375,23 +377,31 @@ __device__ __forceinline__ uint32_t word_tf(uint32_t y, int g) {
 }
 
 // ---------------------------------------------------------------------------
-// Split + forward NTT, register-blocked (lgN >= 3).
+// Split + forward NTT, register-blocked (lgN >= 3, ntt_fast.cuh).
 //
-// 256 threads per CTA.  Small transforms (N <= 2048) are packed several per
-// CTA: a team of N/8 threads owns one entry and each thread the 8 points
-// x = q N/8 + t of the first pass, whose 30-bit coefficient digits it
-// extracts once and keeps in registers for all P primes.  A residue is
+// Team CTAs (N <= 2048): 256 threads, 2048 / N entries; a team of N / 8
+// threads owns one entry and each thread the 8 points x = q N/8 + t of the
+// first pass, whose 30-bit coefficient digits it extracts once and keeps in
+// registers for all its primes.  A residue is
 //     c mod p = REDC( sum_q d_q * (2^(30 q + 32) mod p) )
 // (D products of 30-bit by 30-bit numbers, exact in 64 bits for D <= 8), so
 // each prime costs D wide multiply-adds and one Montgomery reduction instead
-// of a Horner chain.  Larger transforms take a whole CTA; their digits are
-// extracted once into shared memory when it has room (else per prime).  Then
-// passes of 3 stages in registers (ntt_fast.cuh).
+// of a Horner chain.  Larger transforms take a whole CTA of 512 or 1024
+// threads, which extracts a coefficient's digits once for kCtaPrimes primes
+// whose transforms sit in shared memory together.
+//
+// Bound by integer issue: about 58 instructions a residue (2^9 .. 2^11
+// points, 5 digits), the multiply pipe as busy as the issue slots.  With the
+// length a template parameter (addresses and twiddle runs, ntt_fast.cuh),
+// exchanges inside a warp past the first pass and two buffers, a team has one
+// barrier a prime; 64 registers leave four CTAs an SM.  The first 512
+// products of the default batch: 1937 us, 2675 with lengths at run time, a
+// barrier a pass and three CTAs an SM (86 instructions a residue); 1980 at
+// 80 registers.  Few CTAs are cut by primes (prime_chunks): 4 x 4 of
+// 4096-bit entries 10.8 us, 19 with all nine primes in one CTA.
 // ---------------------------------------------------------------------------
 constexpr int kFwdThreads = 256;
-// dynamic shared memory of a whole-CTA forward launch up to which its
-// digits are cached (three CTAs still fit an SM)
-constexpr int kFwdCacheBytes = 72 * 1024;
+constexpr int kTeamWords = pad4(8 * kFwdThreads);  // one buffer of a team CTA
 
 // Digits of the coefficient starting at bit bit0 (r bits of the entry's nw
 // 32-bit words; bits past the entry read as 0).  Bit positions fit 32 bits:
@@ -436,319 +446,346 @@ __device__ __forceinline__ uint32_t digits_residue(const uint32_t (&dg)[D], int 
   return neg ? 3u * p - v : v;
 }
 
-// Where the forward transform leaves point h of prime j of an entry: the
-// plain frequency-contiguous layout (base + j N + h), or, for an operand of a
-// tensor-core product, blocked by kTcTile = 8 frequencies (a 32-byte sector)
-// across the operand's np entries (base + ((j N / 8 + h / 8) np + e) 8 +
-// h mod 8).
-// TILED is a template flag so that plain launches carry none of the
-// blocked layout's state.
-template <bool TILED>
+// Where the forward transform leaves eight points 8 g .. of prime j of an
+// entry: the plain frequency-contiguous layout (base + j N + 8 g), or, for an
+// operand of a tensor-core product, blocked by kTcTile = 8 frequencies (a
+// 32-byte sector) across the operand's np entries (base + ((j N / 8 + g) np +
+// e) 8).  Either way run number j N / 8 + g times one stride.
 struct FwdOut {
   uint32_t* base;
-  uint32_t np, e;
-  int lgN;
-  __device__ __forceinline__ uint32_t* at(int j, uint32_t h) const {
-    if (!TILED) return base + ((uint64_t)j << lgN) + h;
-    const uint64_t tile = ((uint64_t)j << (lgN - kTcTileLg)) + (h >> kTcTileLg);
-    return base + (tile * np + e) * (uint64_t)kTcTile + (h & (kTcTile - 1u));
+  uint32_t stride;
+  __device__ __forceinline__ FwdOut(uint32_t* res, const FwdDesc& d)
+      : base(res + d.res_off + kTcTile * (uint64_t)d.tile_e),
+        stride(d.tile_np ? kTcTile * d.tile_np : kTcTile) {}
+  // reduced from [0, 4p) to [0, p), vector stores
+  __device__ __forceinline__ void store(uint32_t run, uint32_t (&a)[8], uint32_t p) const {
+    static_assert(kTcTile == 8, "a run is one block");
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t v = reduce_2p(a[q], 2 * p);
+      a[q] = min(v, v - p);
+    }
+    uint4* o = reinterpret_cast<uint4*>(base + (uint64_t)run * stride);
+    o[0] = make_uint4(a[0], a[1], a[2], a[3]);
+    o[1] = make_uint4(a[4], a[5], a[6], a[7]);
   }
 };
 
-// 2^L consecutive points h0 .. (h0 a multiple of 2^L) reduced from [0, 4p)
-// to [0, p), vector stores (a run of up to 8 points never crosses a block)
-template <int L, bool TILED>
-__device__ __forceinline__ void store_points(const FwdOut<TILED>& fo, int j, uint32_t h0,
-                                             uint32_t* a, uint32_t p) {
-  static_assert(kTcTile == 8, "vector stores assume 8-frequency blocks");
-  const uint32_t p2 = 2 * p;
-#pragma unroll
-  for (int q = 0; q < (1 << L); ++q) {
-    const uint32_t v = reduce_2p(a[q], p2);
-    a[q] = v >= p ? v - p : v;
+struct NttTables {
+  const uint2* t;
+  __device__ __forceinline__ uint32_t p(int j) const { return c_primes[j].p; }
+  __device__ __forceinline__ const uint2* tw(int j) const { return t + (size_t)j * kTwStride; }
+};
+
+// One entry's coefficients in shared use by the first pass: HZ (at most N/2
+// of them, the usual case: both factors of a product fit in N together): the
+// upper four points of every group are zero, so their digits and residues
+// are skipped and stage 0 only copies.
+struct Coeffs {
+  const uint32_t* w32;
+  uint32_t nw, r, ncoef;
+  bool neg;
+  __device__ __forceinline__ Coeffs(const FwdDesc& d, const uint64_t* __restrict__ limbs) {
+    const uint32_t nl = (uint32_t)(d.size < 0 ? -d.size : d.size);
+    nw = nl < 0x40000000u ? 2u * nl : 0x80000000u;
+    w32 = reinterpret_cast<const uint32_t*>(limbs + d.limb_off);
+    r = d.r;
+    ncoef = d.ncoef;
+    neg = d.size < 0;
   }
-  if (L == 3) {
-    *reinterpret_cast<uint4*>(fo.at(j, h0)) = make_uint4(a[0], a[1], a[2], a[3]);
-    *reinterpret_cast<uint4*>(fo.at(j, h0 + 4)) = make_uint4(a[4], a[5], a[6], a[7]);
-  } else if (L == 2) {
-    *reinterpret_cast<uint4*>(fo.at(j, h0)) = make_uint4(a[0], a[1], a[2], a[3]);
-  } else {
-    *reinterpret_cast<uint2*>(fo.at(j, h0)) = make_uint2(a[0], a[1]);
+  template <int D>
+  __device__ __forceinline__ void digits(int x, uint32_t (&dg)[D]) const {
+    coeff_digits<D>(w32, nw, (uint32_t)x * r, r, (uint32_t)x < ncoef, dg);
   }
+};
+
+// The same value, computed anew as far as the compiler knows: the addresses
+// that follow from it are worth an instruction or two a prime, not a
+// register each across the loop over the primes.
+__device__ __forceinline__ int fresh(int x) {
+  asm volatile("" : "+r"(x));
+  return x;
 }
 
-template <int LP, bool TILED>
-__device__ __forceinline__ void fwd_last_pass(const uint32_t* s, const FwdOut<TILED>& fo, int j,
-                                              bool valid, int lgN, int last_s0, int tt, int TS,
-                                              const uint2* __restrict__ tw, uint32_t p) {
-  for (int g = tt; g < ((1 << lgN) >> LP); g += TS) {
-    uint32_t a[1 << LP];
+// The coefficients of a first-pass group: their digits held in registers for
+// all primes (HZ), or extracted again for every prime (long operands: eight
+// points' digits are too many registers).
+template <int LGN, int D, bool HZ>
+struct FirstGroup {
+  uint32_t dg[HZ ? 4 : 1][D];
+  __device__ __forceinline__ FirstGroup(const Coeffs& co, int g) {
+    if (HZ) {
 #pragma unroll
-    for (int q = 0; q < (1 << LP); ++q) a[q] = s[smi((g << LP) + q)];
-    fwd_group<LP>(a, last_s0, g, tw, p);
-    if (valid) store_points<LP, TILED>(fo, j, (uint32_t)(g << LP), a, p);
-  }
-}
-
-// The body of k_fwd2.  HZ: every polynomial of the CTA has at most N/2
-// coefficients (the usual case: both factors of a product fit in N
-// together), so the first pass's upper four points are zero: their digits
-// and residues are skipped and stage 0 only copies.  dig (whole-CTA HZ
-// transforms, NULL otherwise): shared memory for the entry's digits, digit q
-// of coefficient x at dig[q N/2 + x], extracted once for all P primes.
-template <int D, bool TEAM, bool HZ, bool TILED>
-__device__ __forceinline__ void fwd_body(const FwdDesc& d, uint32_t* s, uint32_t* dig,
-                                         bool valid, int lgN, int P, int tt, int TS,
-                                         const uint64_t* __restrict__ limbs,
-                                         uint32_t* __restrict__ res,
-                                         const uint2* __restrict__ twf) {
-  const int N = 1 << lgN;
-  const uint32_t nl = (uint32_t)(d.size < 0 ? -d.size : d.size);
-  const uint32_t nw = nl < 0x40000000u ? 2u * nl : 0x80000000u;
-  const uint32_t* __restrict__ w32 = reinterpret_cast<const uint32_t*>(limbs + d.limb_off);
-  const bool neg = d.size < 0;
-  const int ng0 = N >> 3;  // groups (and the point stride) of the first pass
-  constexpr int QN = HZ ? 4 : 8;  // points of a first-pass group that can be nonzero
-  const bool cached = !TEAM && HZ && dig != nullptr;
-
-  uint32_t dg[QN][D];
-  if (TEAM) {
-#pragma unroll
-    for (int q = 0; q < QN; ++q) {
-      const int x = q * ng0 + tt;
-      coeff_digits<D>(w32, nw, (uint32_t)x * d.r, d.r, (uint32_t)x < d.ncoef, dg[q]);
+      for (int q = 0; q < 4; ++q) co.digits<D>(q * NttShape<LGN>::NG + g, dg[q]);
     }
-  } else if (cached) {
-    const int half = N >> 1;
-    for (int x = tt; x < half; x += TS) {
-      uint32_t t[D];
-      coeff_digits<D>(w32, nw, (uint32_t)x * d.r, d.r, (uint32_t)x < d.ncoef, t);
-#pragma unroll
-      for (int q = 0; q < D; ++q) dig[q * half + x] = t[q];
-    }
-    __syncthreads();
   }
-  FwdOut<TILED> fo;
-  fo.base = res + d.res_off;
-  fo.np = d.tile_np;
-  fo.e = d.tile_e;
-  fo.lgN = lgN;
-  for (int j = 0; j < P; ++j) {
+  // the group's residues mod prime j through the first pass
+  __device__ __forceinline__ void run(const Coeffs& co, int g, int j,
+                                      const uint2* __restrict__ tw, uint32_t (&a)[8]) {
     const uint32_t p = c_primes[j].p;
-    const uint2* tw = twf + (size_t)j * kTwStride;
-    for (int g = tt; g < ng0; g += TS) {
+    if (HZ) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = digits_residue<D>(dg[q], j, co.neg);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        co.digits<D>(q * NttShape<LGN>::NG + g, dg[0]);
+        a[q] = digits_residue<D>(dg[0], j, co.neg);
+      }
+    }
+    const Tw8 t(tw, 1);
+    if (HZ) {
+      fwd_stage0_upper_zero<3>(a, p);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) bf_fwd(a[q], a[q + 4], t.w1, p, 2 * p);
+    }
+    fwd8<1>(a, t, p);
+  }
+};
+
+template <int LGN, int D, bool HZ>
+__device__ __forceinline__ void fwd_team(const FwdDesc& d, bool valid, uint32_t* sm, int team,
+                                         int tt, int j0, int j1,
+                                         const uint64_t* __restrict__ limbs,
+                                         uint32_t* __restrict__ res, NttTables tables) {
+  using S = NttShape<LGN>;
+  const Coeffs co(d, limbs);
+  const FwdOut out(res, d);
+  FirstGroup<LGN, D, HZ> first(co, tt);
+#pragma unroll 1
+  for (int j = j0; j < j1; ++j) {
+    tt = fresh(tt);
+    const uint32_t p = c_primes[j].p;
+    const uint2* tw = tables.tw(j);
+    // primes alternate between two buffers: a buffer is written again only
+    // after the next prime's barrier, past every thread's last read of it
+    uint32_t* s = sm + pad4(team << LGN) + (j & 1) * kTeamWords;
+    uint32_t a[8];
+    first.run(co, tt, j, tw, a);
+    if constexpr (S::LAST > 0) {
+      store_group<LGN, 0>(s, tt, a);
+      pass_sync<LGN, 0>();
+      fwd_middle<LGN, 3, S::NG>(s, 1, j, tt, tables);
+      load_run(s, tt, a);
+      fwd_tail<LGN>(a, tt, tw, p);
+    }
+    if (valid) out.store((uint32_t)(j * S::NG + tt), a, p);
+  }
+}
+
+// the entry of a team or CTA: items == nullptr: entries 0, 1, .. all alike (u)
+__device__ __forceinline__ CtaItem cta_item(const CtaItem* __restrict__ items,
+                                            const CtaUniform& u) {
+  if (items) return items[blockIdx.x];
+  CtaItem it;
+  const uint32_t g = blockIdx.x / u.chunks, c = blockIdx.x - g * u.chunks;
+  it.first = g * u.per;
+  it.count = (uint16_t)min(u.per, u.total - it.first);
+  it.lgN = (uint8_t)u.lgN;
+  it.j0 = (uint8_t)(u.P * c / u.chunks);
+  it.j1 = (uint8_t)(u.P * (c + 1) / u.chunks);
+  return it;
+}
+
+#define MPZMM_TEAM_SIZES(X) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11)
+
+template <int D>
+__global__ void __launch_bounds__(kFwdThreads, 4)
+k_fwd_team(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
+           const CtaItem* __restrict__ items, CtaUniform u, const uint64_t* __restrict__ limbs,
+           uint32_t* __restrict__ res, const uint2* __restrict__ twf) {
+  __shared__ __align__(16) uint32_t buf[2 * kTeamWords];
+  const CtaItem item = cta_item(items, u);
+  const int lgN = item.lgN;
+  const int team = (int)threadIdx.x >> (lgN - 3);
+  const int tt = (int)threadIdx.x & ((1 << (lgN - 3)) - 1);
+  const bool valid = team < (int)item.count;
+  FwdDesc d{};
+  d.r = 1;
+  if (valid) d = descs[idx ? idx[item.first + team] : item.first + team];
+  // one form for the whole CTA (its barriers must be the same code)
+  const bool hz = __syncthreads_and(d.ncoef <= (1u << lgN >> 1));
+  switch (lgN) {
+#define MPZMM_CASE(L)                                                                         \
+  case L:                                                                                     \
+    if (hz)                                                                                   \
+      fwd_team<L, D, true>(d, valid, buf, team, tt, item.j0, item.j1, limbs, res,             \
+                           NttTables{twf});                                                   \
+    else                                                                                      \
+      fwd_team<L, D, false>(d, valid, buf, team, tt, item.j0, item.j1, limbs, res,            \
+                            NttTables{twf});                                                  \
+    break;
+    MPZMM_TEAM_SIZES(MPZMM_CASE)
+#undef MPZMM_CASE
+  }
+}
+
+// Whole-CTA transforms: threads, and primes whose transforms share the
+// shared memory (their coefficients' digits are extracted once for all).
+__host__ __device__ constexpr int cta_threads(int lgN) { return lgN <= 12 ? 512 : 1024; }
+__host__ __device__ constexpr int cta_primes(int lgN) {
+  return lgN <= 13 ? 5 : (lgN == 14 ? 3 : 1);
+}
+
+// the first pass of primes jb .. jb + nb - 1, into their buffers
+template <int LGN, int D, bool HZ>
+__device__ __forceinline__ void fwd_cta_first(const Coeffs& co, uint32_t* sm, int jb, int nb,
+                                              NttTables tables) {
+  each_group<LGN, cta_threads(LGN)>((int)threadIdx.x, [&](int g) {
+    FirstGroup<LGN, D, HZ> first(co, g);
+#pragma unroll 1
+    for (int c = 0; c < nb; ++c) {
+      const int gc = fresh(g);
+      uint32_t a[8];
+      first.run(co, gc, jb + c, tables.tw(jb + c), a);
+      store_group<LGN, 0>(sm + c * NttShape<LGN>::WORDS, gc, a);
+    }
+  });
+}
+
+template <int LGN, int D>
+__global__ void __launch_bounds__(cta_threads(LGN), 1024 / cta_threads(LGN))
+k_fwd_cta(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
+          const CtaItem* __restrict__ items, CtaUniform u, const uint64_t* __restrict__ limbs,
+          uint32_t* __restrict__ res, const uint2* __restrict__ twf) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  using S = NttShape<LGN>;
+  constexpr int NT = cta_threads(LGN);
+  const CtaItem item = cta_item(items, u);
+  const FwdDesc d = descs[idx ? idx[item.first] : item.first];
+  const Coeffs co(d, limbs);
+  const FwdOut out(res, d);
+  const NttTables tables{twf};
+  const bool hz = d.ncoef <= (uint32_t)(S::N >> 1);
+  const int tid = threadIdx.x, j1 = item.j1;
+  for (int jb = item.j0; jb < j1; jb += cta_primes(LGN)) {
+    const int nb = min(cta_primes(LGN), j1 - jb);
+    if (jb > (int)item.j0) __syncthreads();  // every read of the buffers is done
+    if (hz)
+      fwd_cta_first<LGN, D, true>(co, sm, jb, nb, tables);
+    else
+      fwd_cta_first<LGN, D, false>(co, sm, jb, nb, tables);
+    pass_sync<LGN, 0>();
+    fwd_middle<LGN, 3, NT>(sm, nb, jb, tid, tables);
+    for (int c = 0; c < nb; ++c)
+      each_group<LGN, NT>(tid, [&](int g) {
+        uint32_t a[8];
+        load_run(sm + c * S::WORDS, g, a);
+        fwd_tail<LGN>(a, g, tables.tw(jb + c), c_primes[jb + c].p);
+        out.store((uint32_t)((jb + c) * S::NG + g), a, c_primes[jb + c].p);
+      });
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Inverse NTT, register-blocked (lgN >= 3): the forward passes backwards.
+// Every thread reads its eight consecutive points of the last forward pass
+// straight from global memory with vector loads, and the next prime's are
+// loaded before the current prime's passes run (where a thread has one
+// group), so the loads overlap the arithmetic.  The first forward pass
+// inverted writes straight to global memory, values in [0, 2p).  Bound as the
+// forward: 794 us for the first 512 products of the default batch (40
+// registers, six CTAs an SM), 1137 in the earlier form; a chain step of 64
+// entries of 2^14 points 32 us, 157 before its primes went to CTAs of their
+// own.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void load_points(const uint32_t* src, uint32_t (&a)[8]) {
+  const uint4 u = reinterpret_cast<const uint4*>(src)[0];
+  const uint4 v = reinterpret_cast<const uint4*>(src)[1];
+  a[0] = u.x; a[1] = u.y; a[2] = u.z; a[3] = u.w;
+  a[4] = v.x; a[5] = v.y; a[6] = v.z; a[7] = v.w;
+}
+
+// TS threads of one transform (tt among them); primes alternate between two
+// buffers `next` words apart (0: one buffer, a barrier more).
+template <int LGN, int TS>
+__device__ __forceinline__ void inv_run(uint32_t* __restrict__ io, bool valid, uint32_t* sm,
+                                        int next, int tt, int j0, int j1, NttTables tables) {
+  using S = NttShape<LGN>;
+  constexpr bool ONE = S::NG <= TS;  // a group a thread
+  io += (uint64_t)j0 << LGN;
+  uint32_t nx[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) nx[q] = 0u;
+  if (ONE && valid) load_points(io + 8 * tt, nx);
+#pragma unroll 1
+  for (int j = j0; j < j1; ++j, io += S::N) {
+    const uint32_t p = c_primes[j].p;
+    const uint2* tw = tables.tw(j);
+    uint32_t* s = sm + (j & 1) * next;
+    if constexpr (S::LAST == 0) {  // one pass, global -> registers -> global
       uint32_t a[8];
 #pragma unroll
-      for (int q = 0; q < QN; ++q) {
-        const int x = q * ng0 + g;
-        if (!TEAM) {
-          if (cached) {
-#pragma unroll
-            for (int u = 0; u < D; ++u) dg[q][u] = dig[u * (N >> 1) + x];
-          } else {
-            coeff_digits<D>(w32, nw, (uint32_t)x * d.r, d.r, (uint32_t)x < d.ncoef, dg[q]);
-          }
-        }
-        a[q] = digits_residue<D>(dg[q], j, neg);
-      }
-      if (HZ) {
-        fwd_stage0_upper_zero<3>(a, p);
-        fwd_group<3, 1>(a, 0, 0, tw, p);
-      } else {
-        fwd_group<3>(a, 0, 0, tw, p);
-      }
-      if (lgN == 3) {  // the only pass: eight consecutive points, straight out
-        if (valid) store_points<3, TILED>(fo, j, 0u, a, p);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) s[smi(q * ng0 + g)] = a[q];
-      }
-    }
-    if (lgN == 3) continue;  // uniform per CTA
-    __syncthreads();
-    const int last_s0 = ((lgN - 1) / 3) * 3;
-    for (int s0 = 3; s0 < last_s0; s0 += 3) {
-      smem_pass<3, true>(s, lgN, s0, 3, tt, TS, tw, p);
-      __syncthreads();
-    }
-    // the last pass works on groups of 2^LP consecutive points: reduced and
-    // stored straight from registers with vector stores
-    switch (lgN - last_s0) {
-      case 1: fwd_last_pass<1, TILED>(s, fo, j, valid, lgN, last_s0, tt, TS, tw, p); break;
-      case 2: fwd_last_pass<2, TILED>(s, fo, j, valid, lgN, last_s0, tt, TS, tw, p); break;
-      default: fwd_last_pass<3, TILED>(s, fo, j, valid, lgN, last_s0, tt, TS, tw, p); break;
-    }
-    __syncthreads();  // before the next prime's first pass overwrites s
-  }
-}
-
-// dig_words: shared memory words after the transform reserved for the digit
-// cache of a whole-CTA launch (0: none); it holds D N/2 words for the CTA's
-// transform size.
-template <int D, bool TEAM, bool TILED>
-__global__ void __launch_bounds__(kFwdThreads, 3)
-k_fwd2(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
-       const CtaItem* __restrict__ items, const uint64_t* __restrict__ limbs,
-       uint32_t* __restrict__ res, const uint2* __restrict__ twf, int dig_words) {
-  extern __shared__ uint32_t sm[];
-  const CtaItem item = items[blockIdx.x];
-  const int lgN = item.lgN;
-  const int P = item.P;
-  const int N = 1 << lgN;
-  const int TS = TEAM ? (N >> 3) : kFwdThreads;  // threads per entry
-  const int team = TEAM ? (int)threadIdx.x / TS : 0;
-  const int tt = TEAM ? (int)threadIdx.x % TS : (int)threadIdx.x;
-  const bool valid = team < (int)item.count;
-  uint32_t* s = sm + team * (N + (N >> 5));
-  uint32_t* dig = (!TEAM && dig_words >= D * (N >> 1)) ? s + N + (N >> 5) : nullptr;
-  FwdDesc d;
-  d.limb_off = 0;
-  d.res_off = 0;
-  d.size = 0;
-  d.r = 1;
-  d.ncoef = 0;
-  if (valid) d = descs[idx[item.first + team]];
-  // one variant for the whole CTA (its barriers must be the same code)
-  if (__syncthreads_and(d.ncoef <= (uint32_t)(N >> 1)))
-    fwd_body<D, TEAM, true, TILED>(d, s, dig, valid, lgN, P, tt, TS, limbs, res, twf);
-  else
-    fwd_body<D, TEAM, false, TILED>(d, s, nullptr, valid, lgN, P, tt, TS, limbs, res, twf);
-}
-
-// Inverse NTT, register-blocked (lgN >= 3): the forward passes backwards.
-//
-// The last forward pass (stages last_s0 .. lgN-1, LP = lgN - last_s0 of
-// them) works on groups of 2^LP consecutive points, so its inverse reads
-// each group straight from global memory with one or two vector loads and
-// only then goes to shared memory.  In a team CTA every thread owns exactly
-// eight of those points per prime, and the next prime's eight are loaded
-// into registers before the current prime's passes run, so the loads
-// overlap the arithmetic instead of stalling the warps.
-
-template <int L>
-__device__ __forceinline__ void load_points(const uint32_t* src, uint32_t* a) {
-  if (L == 3) {
-    const uint4 u = *reinterpret_cast<const uint4*>(src);
-    const uint4 v = *reinterpret_cast<const uint4*>(src + 4);
-    a[0] = u.x; a[1] = u.y; a[2] = u.z; a[3] = u.w;
-    a[4] = v.x; a[5] = v.y; a[6] = v.z; a[7] = v.w;
-  } else if (L == 2) {
-    const uint4 u = *reinterpret_cast<const uint4*>(src);
-    a[0] = u.x; a[1] = u.y; a[2] = u.z; a[3] = u.w;
-  } else {
-    const uint2 u = *reinterpret_cast<const uint2*>(src);
-    a[0] = u.x; a[1] = u.y;
-  }
-}
-
-// the groups of the last forward pass (2^LP points each) in registers:
-// inverse stages, then into shared memory
-template <int LP>
-__device__ __forceinline__ void inv_last_pass(uint32_t* s, const uint32_t* a_in, int g,
-                                              int last_s0, const uint2* tw, uint32_t p) {
-  uint32_t a[1 << LP];
-#pragma unroll
-  for (int q = 0; q < (1 << LP); ++q) a[q] = a_in[q];
-  inv_group<LP>(a, last_s0, g, tw, p);
-#pragma unroll
-  for (int q = 0; q < (1 << LP); ++q) s[smi((g << LP) + q)] = a[q];
-}
-
-template <int LP, bool TEAM>
-__device__ __forceinline__ void inv_run(uint32_t* s, uint32_t* __restrict__ res, uint64_t off,
-                                        bool valid, int lgN, int P, int tt, int TS,
-                                        const uint2* __restrict__ twi) {
-  const int N = 1 << lgN;
-  const int last_s0 = lgN - LP;
-  constexpr int GT = 8 >> LP;  // groups per thread in a team CTA
-  uint32_t nx[8];               // team: the next prime's points
-  if (TEAM && valid) {
-#pragma unroll
-    for (int k = 0; k < GT; ++k) load_points<LP>(res + off + ((tt + k * TS) << LP), nx + (k << LP));
-  }
-  for (int j = 0; j < P; ++j) {
-    const uint32_t p = c_primes[j].p;
-    const uint2* tw = twi + (size_t)j * kTwStride;
-    uint32_t* io = res + off + (uint64_t)j * (uint64_t)N;
-    if (last_s0 == 0) {
-      // lgN = 3: one pass, global -> registers -> global
-      if (TEAM && valid) {
-        uint32_t a[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) a[q] = nx[q];
-        if (j + 1 < P) load_points<3>(io + N, nx);
-        inv_group<3>(a, 0, 0, tw, p);
+      for (int q = 0; q < 8; ++q) a[q] = nx[q];
+      if (valid && j + 1 < j1) load_points(io + S::N, nx);
+      inv_tail<LGN>(a, 0, tw, p);
+      if (valid) {
         uint4* o = reinterpret_cast<uint4*>(io);
         o[0] = make_uint4(a[0], a[1], a[2], a[3]);
         o[1] = make_uint4(a[4], a[5], a[6], a[7]);
       }
-      continue;
-    }
-    if (TEAM) {
-      uint32_t a[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) a[q] = valid ? nx[q] : 0u;
-      if (valid && j + 1 < P) {
-#pragma unroll
-        for (int k = 0; k < GT; ++k)
-          load_points<LP>(io + N + ((tt + k * TS) << LP), nx + (k << LP));
-      }
-#pragma unroll
-      for (int k = 0; k < GT; ++k) inv_last_pass<LP>(s, a + (k << LP), tt + k * TS, last_s0, tw, p);
     } else {
-      for (int g = tt; g < (N >> LP); g += TS) {
-        uint32_t a[1 << LP];
-        if (valid) {
-          load_points<LP>(io + (g << LP), a);
+      each_group<LGN, TS>(tt, [&](int g) {
+        uint32_t a[8];
+        if constexpr (ONE) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) a[q] = nx[q];
+          if (valid && j + 1 < j1) load_points(io + S::N + 8 * g, nx);
         } else {
-#pragma unroll
-          for (int q = 0; q < (1 << LP); ++q) a[q] = 0u;
+          load_points(io + 8 * g, a);
         }
-        inv_last_pass<LP>(s, a, g, last_s0, tw, p);
-      }
-    }
-    __syncthreads();
-    for (int s0 = last_s0 - 3; s0 >= 3; s0 -= 3) {
-      smem_pass<3, false>(s, lgN, s0, 3, tt, TS, tw, p);
-      __syncthreads();
-    }
-    // first forward pass (stages 0..2) inverted, straight to global memory
-    for (int g = tt; g < (N >> 3); g += TS) {
-      uint32_t a[8];
+        inv_tail<LGN>(a, g, tw, p);
+        store_run(s, g, a);
+      });
+      inv_middle<LGN, S::LAST - 3, TS>(s, j, tt, tables);
+      const Tw8 t(tw, 1);
+      each_group<LGN, TS>(tt, [&](int g) {
+        uint32_t a[8];
+        load_group<LGN, 0>(s, g, a);
+        inv8(a, t, p);
+        if (valid) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) a[q] = s[smi(q * (N >> 3) + g)];
-      inv_group<3>(a, 0, 0, tw, p);
-      if (valid) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) io[q * (N >> 3) + g] = a[q];  // in [0, 2p)
-      }
+          for (int q = 0; q < 8; ++q) io[q * S::NG + g] = a[q];
+        }
+      });
+      if (next == 0) __syncthreads();
     }
-    __syncthreads();
   }
 }
 
-template <bool TEAM>
-__global__ void __launch_bounds__(kFwdThreads)
-k_inv2(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
-       const CtaItem* __restrict__ items, uint32_t* __restrict__ res,
-       const uint2* __restrict__ twi) {
-  extern __shared__ uint32_t sm[];
-  const CtaItem item = items[blockIdx.x];
+__global__ void __launch_bounds__(kFwdThreads, 6)
+k_inv_team(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
+           const CtaItem* __restrict__ items, CtaUniform u, uint32_t* __restrict__ res,
+           const uint2* __restrict__ twi) {
+  __shared__ __align__(16) uint32_t buf[2 * kTeamWords];
+  const CtaItem item = cta_item(items, u);
   const int lgN = item.lgN;
-  const int P = item.P;
-  const int N = 1 << lgN;
-  const int TS = TEAM ? (N >> 3) : kFwdThreads;
-  const int team = TEAM ? (int)threadIdx.x / TS : 0;
-  const int tt = TEAM ? (int)threadIdx.x % TS : (int)threadIdx.x;
+  const int team = (int)threadIdx.x >> (lgN - 3);
+  const int tt = (int)threadIdx.x & ((1 << (lgN - 3)) - 1);
   const bool valid = team < (int)item.count;
-  uint32_t* s = sm + team * (N + (N >> 5));
-  const uint64_t off = valid ? descs[idx[item.first + team]].res_off : 0;
-  const int last_s0 = ((lgN - 1) / 3) * 3;  // start of the last forward pass
-  switch (lgN - last_s0) {
-    case 1: inv_run<1, TEAM>(s, res, off, valid, lgN, P, tt, TS, twi); break;
-    case 2: inv_run<2, TEAM>(s, res, off, valid, lgN, P, tt, TS, twi); break;
-    default: inv_run<3, TEAM>(s, res, off, valid, lgN, P, tt, TS, twi); break;
+  uint32_t* io = res + (valid ? descs[idx ? idx[item.first + team] : item.first + team].res_off : 0);
+  switch (lgN) {
+#define MPZMM_CASE(L)                                                                      \
+  case L:                                                                                  \
+    inv_run<L, (1 << L) / 8>(io, valid, buf + pad4(team << L), kTeamWords, tt, item.j0,    \
+                             item.j1, NttTables{twi});                                     \
+    break;
+    MPZMM_TEAM_SIZES(MPZMM_CASE)
+#undef MPZMM_CASE
   }
+}
+
+template <int LGN>
+__global__ void __launch_bounds__(cta_threads(LGN), 1024 / cta_threads(LGN))
+k_inv_cta(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
+          const CtaItem* __restrict__ items, CtaUniform u, uint32_t* __restrict__ res,
+          const uint2* __restrict__ twi) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  const CtaItem item = cta_item(items, u);
+  uint32_t* io = res + descs[idx ? idx[item.first] : item.first].res_off;
+  inv_run<LGN, cta_threads(LGN)>(io, true, sm, LGN == 15 ? 0 : NttShape<LGN>::WORDS,
+                                 (int)threadIdx.x, item.j0, item.j1, NttTables{twi});
 }
 
 // ---------------------------------------------------------------------------
@@ -863,8 +900,15 @@ __device__ __forceinline__ void col_last_inv(uint32_t* s, const uint32_t* __rest
   }
 }
 
-// Split + column transforms + twist.  grid = entries x tiles (2 R tiles of
-// W = 2048 / R columns per entry); every entry of a launch has 2^lgN points.
+// primes [P y / Y, P (y + 1) / Y) of grid row y of Y
+__device__ __forceinline__ void chunk_primes(int P, int* j0, int* j1) {
+  *j0 = (int)(P * blockIdx.y / gridDim.y);
+  *j1 = (int)(P * (blockIdx.y + 1) / gridDim.y);
+}
+
+// Split + column transforms + twist.  grid = (entries x tiles, chunks of
+// primes) (2 R tiles of W = 2048 / R columns per entry); every entry of a
+// launch has 2^lgN points.
 template <int D>
 __global__ void __launch_bounds__(kFwdThreads, 3)
 k_fwd_cols(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx, int tiles,
@@ -897,7 +941,9 @@ k_fwd_cols(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx, 
     coeff_digits<D>(w32, nw, x * d.r, d.r, x < d.ncoef && !(hz && k >= 4), dg[k]);
   }
   const int last_s0 = ((lgR - 1) / 3) * 3;
-  for (int j = 0; j < (int)d.P; ++j) {
+  int j0, j1;
+  chunk_primes(d.P, &j0, &j1);
+  for (int j = j0; j < j1; ++j) {
     const uint32_t p = c_primes[j].p;
     const uint2* tw = twf + (size_t)j * kTwStride;
     uint32_t a[8];
@@ -931,16 +977,21 @@ k_fwd_cols(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx, 
   }
 }
 
-// C-point transforms of the blocks.  grid = entries x R blocks.  Forward:
-// ordinary forward transform of each (twisted) block.  Inverse: ordinary
-// inverse transform, then the untwist psi_b^-y (tt holds the inverse twist
-// tables).  Descriptors: fdescs (forward) or idescs (inverse).
+// C-point transforms of the blocks.  grid = (entries x R blocks, chunks of
+// primes).  Forward: ordinary forward transform of each (twisted) block.
+// Inverse: ordinary inverse transform, then the untwist psi_b^-y (tt holds
+// the inverse twist tables).  Descriptors: fdescs (forward) or idescs
+// (inverse).  Two buffers in turn, as the team kernels.
+constexpr int kBlockThreads = 1 << (kLargeLgC - 3);  // a group of eight a thread
+
 template <bool FWD>
-__global__ void __launch_bounds__(kFwdThreads)
+__global__ void __launch_bounds__(kBlockThreads, 2)
 k_ntt_blocks(const FwdDesc* __restrict__ fdescs, const InvDesc* __restrict__ idescs,
              const uint32_t* __restrict__ idx, int blocks, uint32_t* __restrict__ res,
              const uint2* __restrict__ tws, TwistTab tt) {
-  extern __shared__ uint32_t sm[];
+  constexpr int lgC = kLargeLgC;
+  using S = NttShape<lgC>;
+  __shared__ __align__(16) uint32_t buf[2 * S::WORDS];
   const int e = blockIdx.x / blocks;
   const int b = blockIdx.x - e * blocks;
   uint64_t off;
@@ -956,71 +1007,53 @@ k_ntt_blocks(const FwdDesc* __restrict__ fdescs, const InvDesc* __restrict__ ide
     lgN = d.lgN;
     P = d.P;
   }
-  constexpr int lgC = kLargeLgC;
-  constexpr int C = 1 << lgC;
-  constexpr int last_s0 = ((lgC - 1) / 3) * 3;
-  static_assert(lgC - last_s0 == 3, "the block length must end on a full pass");
   const int lgR = lgN - lgC;
   const uint64_t N = (uint64_t)1 << lgN;
   const int tid = threadIdx.x;
   const uint32_t bb = __brev((uint32_t)b) >> (32 - lgR);
-  for (int j = 0; j < P; ++j) {
+  const NttTables tables{tws};
+  int j0, j1;
+  chunk_primes(P, &j0, &j1);
+#pragma unroll 1
+  for (int j = j0; j < j1; ++j) {
     const uint32_t p = c_primes[j].p;
-    const uint2* tw = tws + (size_t)j * kTwStride;
+    const uint2* tw = tables.tw(j);
     uint32_t* io = res + off + (uint64_t)j * N + ((uint64_t)b << lgC);
+    uint32_t* s = buf + (j & 1) * S::WORDS;
+    uint32_t a[8];
     if (FWD) {
-      for (int v = tid; v < C / 4; v += kFwdThreads) {
-        const uint4 u = reinterpret_cast<const uint4*>(io)[v];
-        sm[smi(4 * v)] = u.x;
-        sm[smi(4 * v + 1)] = u.y;
-        sm[smi(4 * v + 2)] = u.z;
-        sm[smi(4 * v + 3)] = u.w;
-      }
-      __syncthreads();
-      for (int s0 = 0; s0 < last_s0; s0 += 3) {
-        smem_pass<3, true>(sm, lgC, s0, 3, tid, kFwdThreads, tw, p);
-        __syncthreads();
-      }
-      // a four-step block: plain layout, the block's points from b C on
-      FwdOut<false> fo;
-      fo.base = res + off + ((uint64_t)b << lgC);
-      fo.np = 0;
-      fo.e = 0;
-      fo.lgN = lgN;
-      fwd_last_pass<3>(sm, fo, j, true, lgC, last_s0, tid, kFwdThreads, tw, p);
-      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] = io[q * S::NG + tid];
+      fwd8(a, Tw8(tw, 1), p);
+      store_group<lgC, 0>(s, tid, a);
+      pass_sync<lgC, 0>();
+      fwd_middle<lgC, 3, kBlockThreads>(s, 1, j, tid, tables);
+      load_run(s, tid, a);
+      fwd_tail<lgC>(a, tid, tw, p);
+      FwdDesc d{};
+      d.res_off = off + (uint64_t)j * N + ((uint64_t)b << lgC);
+      FwdOut(res, d).store((uint32_t)tid, a, p);
     } else {
-      for (int g = tid; g < C / 8; g += kFwdThreads) {
-        uint32_t a[8];
-        load_points<3>(io + (g << 3), a);
-        inv_last_pass<3>(sm, a, g, last_s0, tw, p);
-      }
-      __syncthreads();
-      for (int s0 = last_s0 - 3; s0 >= 3; s0 -= 3) {
-        smem_pass<3, false>(sm, lgC, s0, 3, tid, kFwdThreads, tw, p);
-        __syncthreads();
-      }
+      load_points(io + 8 * tid, a);
+      inv_tail<lgC>(a, tid, tw, p);
+      store_run(s, tid, a);
+      inv_middle<lgC, S::LAST - 3, kBlockThreads>(s, j, tid, tables);
+      load_group<lgC, 0>(s, tid, a);
+      inv8(a, Tw8(tw, 1), p);
       const uint2* th = tt.hi + (size_t)j * kTwistEntries;
       const uint32_t* tl = tt.lo + (size_t)j * kTwistEntries;
       const uint32_t pinv = c_primes[j].pinv;
-      for (int g = tid; g < C / 8; g += kFwdThreads) {
-        uint32_t a[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) a[q] = sm[smi(q * (C / 8) + g)];
-        inv_group<3>(a, 0, 0, tw, p);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const uint32_t y = (uint32_t)(q * (C / 8) + g);
-          io[y] = twist_mul(a[q], (bb * y) << (20 - lgN), th, tl, p, pinv);
-        }
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t y = (uint32_t)(q * S::NG + tid);
+        io[y] = twist_mul(a[q], (bb * y) << (20 - lgN), th, tl, p, pinv);
       }
-      __syncthreads();
     }
   }
 }
 
 // Inverse column transforms, natural coefficient order out (values in
-// [0, 2p), as the CRT expects).  grid = entries x tiles, as k_fwd_cols.
+// [0, 2p), as the CRT expects).  grid as k_fwd_cols.
 __global__ void __launch_bounds__(kFwdThreads)
 k_inv_cols(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx, int tiles,
            uint32_t* __restrict__ res, const uint2* __restrict__ twi) {
@@ -1037,7 +1070,9 @@ k_inv_cols(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx, 
   const int g = (int)threadIdx.x >> lgW;
   const int lgR8 = lgR - 3;
   const int last_s0 = ((lgR - 1) / 3) * 3;
-  for (int j = 0; j < (int)d.P; ++j) {
+  int j0, j1;
+  chunk_primes(d.P, &j0, &j1);
+  for (int j = j0; j < j1; ++j) {
     const uint32_t p = c_primes[j].p;
     const uint2* tw = twi + (size_t)j * kTwStride;
     uint32_t* io = res + d.res_off + (uint64_t)j * N;
@@ -2066,88 +2101,100 @@ static int ntt_threads(int lgN) {
   return half < 32 ? 32 : (half > 1024 ? 1024 : half);
 }
 
-template <int D, bool TILED>
-static cudaError_t launch_fwd2_d(const FwdDesc* descs, const uint32_t* idx,
-                                 const CtaItem* items, int nitems, bool team, int max_lgN,
-                                 const uint64_t* limbs, uint32_t* res, const uint2* twf,
-                                 cudaStream_t st) {
-  const int Nmax = 1 << max_lgN;
-  if (team) {
-    const size_t smem = sizeof(uint32_t) * (size_t)(8 * kFwdThreads + (8 * kFwdThreads >> 5));
-    k_fwd2<D, true, TILED><<<nitems, kFwdThreads, smem, st>>>(descs, idx, items, limbs, res, twf, 0);
-  } else {
-    // whole-CTA transforms: the digit cache when the launch still fits
-    // three CTAs an SM with it (every CTA's transform is at most Nmax)
-    size_t smem = sizeof(uint32_t) * (size_t)(Nmax + (Nmax >> 5));
-    const size_t cache = sizeof(uint32_t) * (size_t)D * (size_t)(Nmax >> 1);
-    int dig_words = 0;
-    if (smem + cache <= (size_t)kFwdCacheBytes) {
-      smem += cache;
-      dig_words = D * (Nmax >> 1);
-    }
-    k_fwd2<D, false, TILED><<<nitems, kFwdThreads, smem, st>>>(descs, idx, items, limbs, res, twf,
-                                                        dig_words);
+int fwd_team_points() { return 8 * kFwdThreads; }
+
+#define MPZMM_CTA_SIZES(X) X(12) X(13) X(14) X(15)
+#define MPZMM_DIGITS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
+
+// dynamic shared memory of a whole-CTA launch whose CTAs have up to `primes`
+static size_t fwd_cta_bytes(int lgN, int primes) {
+  return sizeof(uint32_t) * (size_t)pad4(1 << lgN) * (size_t)std::min(primes, cta_primes(lgN));
+}
+static size_t inv_cta_bytes(int lgN) {
+  return sizeof(uint32_t) * (size_t)pad4(1 << lgN) * (lgN == 15 ? 1 : 2);
+}
+
+template <int D>
+static cudaError_t launch_fwd_d(const FwdDesc* descs, const uint32_t* idx, const CtaItem* items,
+                                int nitems, CtaUniform u, int lgN, int primes,
+                                const uint64_t* limbs, uint32_t* res, const uint2* twf,
+                                cudaStream_t st) {
+  switch (lgN) {
+#define MPZMM_CASE(L)                                                                           \
+  case L:                                                                                       \
+    k_fwd_cta<L, D><<<nitems, cta_threads(L), fwd_cta_bytes(L, primes), st>>>(descs, idx,       \
+                                                                              items, u, limbs,  \
+                                                                              res, twf);        \
+    break;
+    MPZMM_CTA_SIZES(MPZMM_CASE)
+#undef MPZMM_CASE
+    default:
+      k_fwd_team<D><<<nitems, kFwdThreads, 0, st>>>(descs, idx, items, u, limbs, res, twf);
   }
   return cudaGetLastError();
 }
 
-int fwd_team_points() { return 8 * kFwdThreads; }
-
-template <bool TILED>
-static cudaError_t launch_fwd_items_t(const FwdDesc* descs, const uint32_t* idx,
-                                      const CtaItem* items, int nitems, int D, bool team,
-                                      int max_lgN, const uint64_t* limbs, uint32_t* res,
-                                      const uint2* twf, cudaStream_t st) {
+static cudaError_t launch_fwd(const FwdDesc* descs, const uint32_t* idx, const CtaItem* items,
+                              int nitems, CtaUniform u, int D, int lgN, int primes,
+                              const uint64_t* limbs, uint32_t* res, const uint2* twf,
+                              cudaStream_t st) {
+  if (nitems == 0) return cudaSuccess;
   switch (D) {
-#define MPZMM_FWD_CASE(DD) \
-  case DD:                 \
-    return launch_fwd2_d<DD, TILED>(descs, idx, items, nitems, team, max_lgN, limbs, res, twf, st);
-    MPZMM_FWD_CASE(1)
-    MPZMM_FWD_CASE(2)
-    MPZMM_FWD_CASE(3)
-    MPZMM_FWD_CASE(4)
-    MPZMM_FWD_CASE(5)
-    MPZMM_FWD_CASE(6)
-    MPZMM_FWD_CASE(7)
-#undef MPZMM_FWD_CASE
+#define MPZMM_CASE(DD) \
+  case DD:             \
+    return launch_fwd_d<DD>(descs, idx, items, nitems, u, lgN, primes, limbs, res, twf, st);
+    MPZMM_DIGITS(MPZMM_CASE)
+#undef MPZMM_CASE
     default:
       return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t launch_fwd_items(const FwdDesc* descs, const uint32_t* idx, const CtaItem* items,
-                             int nitems, int D, bool team, int max_lgN, const uint64_t* limbs,
-                             uint32_t* res, const uint2* twf, cudaStream_t st, bool tiled) {
+static cudaError_t launch_inv(const InvDesc* descs, const uint32_t* idx, const CtaItem* items,
+                              int nitems, CtaUniform u, int lgN, uint32_t* res,
+                              const uint2* twi, cudaStream_t st) {
   if (nitems == 0) return cudaSuccess;
-  return tiled ? launch_fwd_items_t<true>(descs, idx, items, nitems, D, team, max_lgN, limbs, res,
-                                         twf, st)
-               : launch_fwd_items_t<false>(descs, idx, items, nitems, D, team, max_lgN, limbs,
-                                          res, twf, st);
+  switch (lgN) {
+#define MPZMM_CASE(L)                                                                      \
+  case L:                                                                                  \
+    k_inv_cta<L><<<nitems, cta_threads(L), inv_cta_bytes(L), st>>>(descs, idx, items, u, res, \
+                                                                   twi);                   \
+    break;
+    MPZMM_CTA_SIZES(MPZMM_CASE)
+#undef MPZMM_CASE
+    default:
+      k_inv_team<<<nitems, kFwdThreads, 0, st>>>(descs, idx, items, u, res, twi);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fwd_items(const FwdDesc* descs, const uint32_t* idx, const CtaItem* items,
+                             int nitems, int D, bool team, int max_lgN, int primes,
+                             const uint64_t* limbs, uint32_t* res, const uint2* twf,
+                             cudaStream_t st) {
+  return launch_fwd(descs, idx, items, nitems, CtaUniform{}, D, team ? 0 : max_lgN, primes, limbs,
+                    res, twf, st);
 }
 
 cudaError_t launch_inv_items(const InvDesc* descs, const uint32_t* idx, const CtaItem* items,
                              int nitems, bool team, int max_lgN, uint32_t* res,
                              const uint2* twi, cudaStream_t st) {
-  if (nitems == 0) return cudaSuccess;
-  const int Nmax = 1 << max_lgN;
-  const size_t smem = team ? sizeof(uint32_t) * (size_t)(8 * kFwdThreads + (8 * kFwdThreads >> 5))
-                           : sizeof(uint32_t) * (size_t)(Nmax + (Nmax >> 5));
-  if (team) {
-    k_inv2<true><<<nitems, kFwdThreads, smem, st>>>(descs, idx, items, res, twi);
-  } else {
-    k_inv2<false><<<nitems, kFwdThreads, smem, st>>>(descs, idx, items, res, twi);
-  }
-  return cudaGetLastError();
+  return launch_inv(descs, idx, items, nitems, CtaUniform{}, team ? 0 : max_lgN, res, twi, st);
 }
 
-// shared memory of the four-step kernels
-static size_t col_tile_bytes() { return sizeof(uint32_t) * (size_t)(kColPoints + (kColPoints >> 5)); }
-static size_t block_bytes() {
-  return sizeof(uint32_t) * (size_t)((1 << kLargeLgC) + ((1 << kLargeLgC) >> 5));
+// Chunks of primes a transform's CTAs take each, when there are `ctas`
+// whole ones: one while those give every SM two, else as many as do.
+int prime_chunks(uint64_t ctas, int P, int sms) {
+  const uint64_t want = 2 * (uint64_t)(sms > 0 ? sms : 1);
+  if (ctas == 0 || ctas >= want) return 1;
+  return (int)std::min<uint64_t>((uint64_t)P, (want + ctas - 1) / ctas);
 }
+
+// shared memory of a column tile of the four-step kernels
+static size_t col_tile_bytes() { return sizeof(uint32_t) * (size_t)(kColPoints + (kColPoints >> 5)); }
 
 template <int D>
-static void launch_fwd_cols_d(int grid, cudaStream_t st, const FwdDesc* descs, const uint32_t* idx,
+static void launch_fwd_cols_d(dim3 grid, cudaStream_t st, const FwdDesc* descs, const uint32_t* idx,
                               int tiles, const uint64_t* limbs, uint32_t* res, const uint2* twf,
                               const TwistTab& tt) {
   k_fwd_cols<D><<<grid, kFwdThreads, col_tile_bytes(), st>>>(descs, idx, tiles, limbs, res, twf,
@@ -2156,14 +2203,14 @@ static void launch_fwd_cols_d(int grid, cudaStream_t st, const FwdDesc* descs, c
 
 int large_tiles(int lgN) { return 1 << (lgN - kLargeLgC + 1); }
 
-cudaError_t launch_large_fwd(const FwdDesc* descs, const uint32_t* idx, int count, int lgN, int D,
-                             const uint64_t* limbs, uint32_t* res, const uint2* twf,
+cudaError_t launch_large_fwd(const FwdDesc* descs, const uint32_t* idx, int count, int lgN, int P,
+                             int D, int sms, const uint64_t* limbs, uint32_t* res, const uint2* twf,
                              const TwistTab& tt, cudaStream_t st) {
   if (count == 0) return cudaSuccess;
   if (lgN <= kMaxLgNOneCta || lgN > kMaxLgN) return cudaErrorInvalidValue;
   const int tiles = large_tiles(lgN);
   const int blocks = 1 << (lgN - kLargeLgC);
-  const int grid = count * tiles;
+  const dim3 grid(count * tiles, prime_chunks((uint64_t)count * tiles, P, sms));
   switch (D) {
     case 1: launch_fwd_cols_d<1>(grid, st, descs, idx, tiles, limbs, res, twf, tt); break;
     case 2: launch_fwd_cols_d<2>(grid, st, descs, idx, tiles, limbs, res, twf, tt); break;
@@ -2176,23 +2223,24 @@ cudaError_t launch_large_fwd(const FwdDesc* descs, const uint32_t* idx, int coun
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_ntt_blocks<true><<<count * blocks, kFwdThreads, block_bytes(), st>>>(descs, nullptr, idx,
-                                                                         blocks, res, twf, tt);
+  const dim3 bgrid(count * blocks, prime_chunks((uint64_t)count * blocks, P, sms));
+  k_ntt_blocks<true><<<bgrid, kBlockThreads, 0, st>>>(descs, nullptr, idx, blocks, res, twf, tt);
   return cudaGetLastError();
 }
 
-cudaError_t launch_large_inv(const InvDesc* descs, const uint32_t* idx, int count, int lgN,
-                             uint32_t* res, const uint2* twi, const TwistTab& tt,
+cudaError_t launch_large_inv(const InvDesc* descs, const uint32_t* idx, int count, int lgN, int P,
+                             int sms, uint32_t* res, const uint2* twi, const TwistTab& tt,
                              cudaStream_t st) {
   if (count == 0) return cudaSuccess;
   if (lgN <= kMaxLgNOneCta || lgN > kMaxLgN) return cudaErrorInvalidValue;
   const int tiles = large_tiles(lgN);
   const int blocks = 1 << (lgN - kLargeLgC);
-  k_ntt_blocks<false><<<count * blocks, kFwdThreads, block_bytes(), st>>>(nullptr, descs, idx,
-                                                                          blocks, res, twi, tt);
+  const dim3 bgrid(count * blocks, prime_chunks((uint64_t)count * blocks, P, sms));
+  k_ntt_blocks<false><<<bgrid, kBlockThreads, 0, st>>>(nullptr, descs, idx, blocks, res, twi, tt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_inv_cols<<<count * tiles, kFwdThreads, col_tile_bytes(), st>>>(descs, idx, tiles, res, twi);
+  const dim3 grid(count * tiles, prime_chunks((uint64_t)count * tiles, P, sms));
+  k_inv_cols<<<grid, kFwdThreads, col_tile_bytes(), st>>>(descs, idx, tiles, res, twi);
   return cudaGetLastError();
 }
 
@@ -2526,40 +2574,25 @@ cudaError_t launch_crt_uniform(const InvDesc* descs, int count, CrtUniform u, in
 // Dynamic shared memory limits of every kernel, set once per device at
 // set-up (so that launches, including those captured into a CUDA graph,
 // issue nothing but stream work).
-template <int D>
-static cudaError_t set_fwd_attrs() {
-  const int big =
-      (int)(sizeof(uint32_t) * ((1 << kMaxLgNOneCta) + ((1 << kMaxLgNOneCta) >> 5)));
-  cudaError_t e;
-  for (auto fn : {k_fwd2<D, true, false>, k_fwd2<D, false, false>, k_fwd2<D, true, true>,
-                  k_fwd2<D, false, true>})
-    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, big)) !=
-        cudaSuccess)
-      return e;
-  return cudaSuccess;
+template <class K>
+static cudaError_t allow_smem(K kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 cudaError_t init_kernel_attributes() {
   cudaError_t e;
-  const int big =
-      (int)(sizeof(uint32_t) * ((1 << kMaxLgNOneCta) + ((1 << kMaxLgNOneCta) >> 5)));
-  if ((e = cudaFuncSetAttribute(k_split_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(uint32_t) << kMaxLgNOneCta))) != cudaSuccess)
+  if ((e = allow_smem(k_split_fwd, sizeof(uint32_t) << kMaxLgNOneCta)) != cudaSuccess ||
+      (e = allow_smem(k_inv_ntt, sizeof(uint32_t) << kMaxLgNOneCta)) != cudaSuccess)
     return e;
-  if ((e = cudaFuncSetAttribute(k_inv_ntt, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(uint32_t) << kMaxLgNOneCta))) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(k_inv2<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)) !=
-      cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(k_inv2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)) !=
-      cudaSuccess)
-    return e;
-  if ((e = set_fwd_attrs<1>()) != cudaSuccess || (e = set_fwd_attrs<2>()) != cudaSuccess ||
-      (e = set_fwd_attrs<3>()) != cudaSuccess || (e = set_fwd_attrs<4>()) != cudaSuccess ||
-      (e = set_fwd_attrs<5>()) != cudaSuccess || (e = set_fwd_attrs<6>()) != cudaSuccess ||
-      (e = set_fwd_attrs<7>()) != cudaSuccess)
-    return e;
+#define MPZMM_FWD(L, D) \
+  if ((e = allow_smem(k_fwd_cta<L, D>, fwd_cta_bytes(L, kMaxPrimes))) != cudaSuccess) return e;
+#define MPZMM_CASE(L)                                                                 \
+  if ((e = allow_smem(k_inv_cta<L>, inv_cta_bytes(L))) != cudaSuccess) return e;      \
+  MPZMM_FWD(L, 1) MPZMM_FWD(L, 2) MPZMM_FWD(L, 3) MPZMM_FWD(L, 4) MPZMM_FWD(L, 5)     \
+  MPZMM_FWD(L, 6) MPZMM_FWD(L, 7)
+  MPZMM_CTA_SIZES(MPZMM_CASE)
+#undef MPZMM_CASE
+#undef MPZMM_FWD
   for (auto fn : {k_crt_mixed<2, kCrtMixedSplit, false>, k_crt_mixed<2, kCrtMixedSplit, true>,
                   k_crt_mixed<kCrtMixedSplit + 1, kMaxPrimes, false>,
                   k_crt_mixed<kCrtMixedSplit + 1, kMaxPrimes, true>})

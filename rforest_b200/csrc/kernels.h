@@ -23,29 +23,32 @@ cudaError_t launch_inv_ntt(const InvDesc* descs, const uint32_t* idx, int count,
 
 // Register-blocked transforms (lgN >= 3) over CTA work items of mixed size
 // classes in ONE launch.  team: every item has 2^lgN <= fwd_team_points()
-// (several entries per CTA); otherwise one entry per CTA and max_lgN sizes
-// the shared memory.  D = digits of 30 bits of the widest coefficient.
+// (several entries per CTA); otherwise one entry of 2^max_lgN points per CTA,
+// with up to `primes` primes.  D = digits of 30 bits of the widest
+// coefficient.  Operands of tensor-core products (FwdDesc::tile_np) are
+// written in the frequency-blocked layout, others in the plain one.
 int fwd_team_points();
-// tiled: the launch's entries are operands of tensor-core products, written
-// in the frequency-blocked layout (FwdDesc::tile_np); else the plain layout.
 cudaError_t launch_fwd_items(const FwdDesc* descs, const uint32_t* idx, const CtaItem* items,
-                             int nitems, int D, bool team, int max_lgN, const uint64_t* limbs,
-                             uint32_t* res, const uint2* twf, cudaStream_t st,
-                             bool tiled = false);
+                             int nitems, int D, bool team, int max_lgN, int primes,
+                             const uint64_t* limbs, uint32_t* res, const uint2* twf,
+                             cudaStream_t st);
 cudaError_t launch_inv_items(const InvDesc* descs, const uint32_t* idx, const CtaItem* items,
                              int nitems, bool team, int max_lgN, uint32_t* res,
                              const uint2* twi, cudaStream_t st);
+// Chunks a launch of `ctas` transform CTAs cuts its P primes into.
+int prime_chunks(uint64_t ctas, int P, int sms);
 
 // Transforms of 2^16 .. 2^20 points (four-step: column transforms, twist,
 // block transforms), `count` entries of one length 2^lgN in one group (idx
 // lists their descriptors).  Forward: split of D-digit coefficients + the
 // transform; inverse: the transform back to natural order, ready for the
-// CRT.  Two launches each.  tt: the twist tables of the direction.
-cudaError_t launch_large_fwd(const FwdDesc* descs, const uint32_t* idx, int count, int lgN, int D,
-                             const uint64_t* limbs, uint32_t* res, const uint2* twf,
+// CRT.  Two launches each (P primes, cut into chunks where the CTAs are
+// few).  tt: the twist tables of the direction.
+cudaError_t launch_large_fwd(const FwdDesc* descs, const uint32_t* idx, int count, int lgN, int P,
+                             int D, int sms, const uint64_t* limbs, uint32_t* res, const uint2* twf,
                              const TwistTab& tt, cudaStream_t st);
-cudaError_t launch_large_inv(const InvDesc* descs, const uint32_t* idx, int count, int lgN,
-                             uint32_t* res, const uint2* twi, const TwistTab& tt,
+cudaError_t launch_large_inv(const InvDesc* descs, const uint32_t* idx, int count, int lgN, int P,
+                             int sms, uint32_t* res, const uint2* twi, const TwistTab& tt,
                              cudaStream_t st);
 constexpr int kLargeLaunches = 2;  // kernel launches per direction of a four-step group
 

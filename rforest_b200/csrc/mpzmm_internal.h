@@ -138,13 +138,21 @@ struct TcItem {
 };
 
 // Work item of one CTA of the batched transform kernels: `count` entries of
-// one size class (all 2^lgN points, P primes), descriptor indices
-// idx[first .. first + count).
+// one size class (all 2^lgN points), descriptor indices
+// idx[first .. first + count), and their primes j0 .. j1 - 1.
 struct CtaItem {
   uint32_t first;
   uint16_t count;
   uint8_t lgN;
-  uint8_t P;
+  uint8_t j0, j1;
+  uint8_t pad[3];
+};
+
+// Entries 0 .. total - 1 that are all alike: `per` a CTA, their P primes in
+// `chunks` CTAs.
+struct CtaUniform {
+  uint32_t total = 0, per = 1, chunks = 1;
+  int lgN = 0, P = 0;
 };
 
 // Work item of one warp of the CRT kernel: words [w0, w1) of output entry
