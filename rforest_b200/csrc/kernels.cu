@@ -108,7 +108,7 @@ __global__ void k_split_fwd(const FwdDesc* __restrict__ descs,
                             uint32_t* __restrict__ res,
                             const uint2* __restrict__ twf) {
   extern __shared__ uint32_t sm[];
-  const FwdDesc d = descs[idx[blockIdx.x]];
+  const FwdDesc d = descs[idx ? idx[blockIdx.x] : blockIdx.x];
   const int j = blockIdx.y;
   const uint32_t p = c_primes[j].p;
   const uint32_t mu = c_primes[j].mu;
@@ -156,7 +156,7 @@ __global__ void k_inv_ntt(const InvDesc* __restrict__ descs,
                           const uint32_t* __restrict__ idx, uint32_t* __restrict__ res,
                           const uint2* __restrict__ twi) {
   extern __shared__ uint32_t sm[];
-  const InvDesc d = descs[idx[blockIdx.x]];
+  const InvDesc d = descs[idx ? idx[blockIdx.x] : blockIdx.x];
   const int j = blockIdx.y;
   const uint32_t p = c_primes[j].p;
   const int N = 1 << d.lgN;
@@ -2188,6 +2188,39 @@ int prime_chunks(uint64_t ctas, int P, int sms) {
   const uint64_t want = 2 * (uint64_t)(sms > 0 ? sms : 1);
   if (ctas == 0 || ctas >= want) return 1;
   return (int)std::min<uint64_t>((uint64_t)P, (want + ctas - 1) / ctas);
+}
+
+// entries 0 .. total - 1 alike: CTAs of `per`, their primes in chunks
+static CtaUniform cta_uniform(uint32_t total, int lgN, int P, int sms, int* nitems, int* primes) {
+  CtaUniform u;
+  u.total = total;
+  u.per = (uint32_t)std::max(1, fwd_team_points() >> lgN);
+  u.lgN = lgN;
+  u.P = P;
+  const uint32_t ctas = (total + u.per - 1) / u.per;
+  u.chunks = (uint32_t)prime_chunks(ctas, P, sms);
+  *nitems = (int)(ctas * u.chunks);
+  *primes = (P + (int)u.chunks - 1) / (int)u.chunks;
+  return u;
+}
+
+cudaError_t launch_fwd_uniform(const FwdDesc* descs, uint32_t total, int lgN, int P, int D,
+                               int sms, const uint64_t* limbs, uint32_t* res, const uint2* twf,
+                               cudaStream_t st) {
+  if (total == 0) return cudaSuccess;
+  if (lgN < 3) return launch_split_fwd(descs, nullptr, (int)total, P, lgN, limbs, res, twf, st);
+  int nitems, primes;
+  const CtaUniform u = cta_uniform(total, lgN, P, sms, &nitems, &primes);
+  return launch_fwd(descs, nullptr, nullptr, nitems, u, D, lgN, primes, limbs, res, twf, st);
+}
+
+cudaError_t launch_inv_uniform(const InvDesc* descs, uint32_t total, int lgN, int P, int sms,
+                               uint32_t* res, const uint2* twi, cudaStream_t st) {
+  if (total == 0) return cudaSuccess;
+  if (lgN < 3) return launch_inv_ntt(descs, nullptr, (int)total, P, lgN, res, twi, st);
+  int nitems, primes;
+  const CtaUniform u = cta_uniform(total, lgN, P, sms, &nitems, &primes);
+  return launch_inv(descs, nullptr, nullptr, nitems, u, lgN, res, twi, st);
 }
 
 // shared memory of a column tile of the four-step kernels

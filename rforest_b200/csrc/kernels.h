@@ -14,7 +14,8 @@ cudaError_t upload_constants(const PrimeConst* primes, const CrtConst* crt);
 cudaError_t init_kernel_attributes();
 
 // Radix-2 split + forward NTT / inverse NTT, one CTA per (entry, prime),
-// for `count` entries of one class (any lgN >= 1; used for lgN < 3).
+// for `count` entries of one class (any lgN >= 1; used for lgN < 3); idx ==
+// nullptr: entries 0, 1, ...
 cudaError_t launch_split_fwd(const FwdDesc* descs, const uint32_t* idx, int count, int P,
                              int lgN, const uint64_t* limbs, uint32_t* res,
                              const uint2* twf, cudaStream_t st);
@@ -35,6 +36,13 @@ cudaError_t launch_fwd_items(const FwdDesc* descs, const uint32_t* idx, const Ct
 cudaError_t launch_inv_items(const InvDesc* descs, const uint32_t* idx, const CtaItem* items,
                              int nitems, bool team, int max_lgN, uint32_t* res,
                              const uint2* twi, cudaStream_t st);
+// The same over entries 0 .. total - 1 that are all alike, without lists (any
+// lgN up to one CTA's).
+cudaError_t launch_fwd_uniform(const FwdDesc* descs, uint32_t total, int lgN, int P, int D,
+                               int sms, const uint64_t* limbs, uint32_t* res, const uint2* twf,
+                               cudaStream_t st);
+cudaError_t launch_inv_uniform(const InvDesc* descs, uint32_t total, int lgN, int P, int sms,
+                               uint32_t* res, const uint2* twi, cudaStream_t st);
 // Chunks a launch of `ctas` transform CTAs cuts its P primes into.
 int prime_chunks(uint64_t ctas, int P, int sms);
 

@@ -159,15 +159,15 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
 
   const int P = prm.P, lgN = prm.lgN, r = prm.r;
   const uint64_t N = (uint64_t)1 << lgN, poly = (uint64_t)P * N;
-  // descriptor blob: fwd (A then B), inv, prod, index lists; the limits
-  // below count 12 bytes for each 128 frequencies of a prime besides
+  // descriptor blob: fwd (A then B), inv, prod; the limits below count 12
+  // bytes for each 128 frequencies of a prime and 4 for each entry besides
   const size_t off_fwd = 0;
   const size_t off_inv = align256(off_fwd + sizeof(FwdDesc) * (size_t)(na + nb));
   const size_t off_pd = align256(off_inv + sizeof(InvDesc) * (size_t)nc);
-  const size_t off_idx = align256(off_pd + sizeof(ProdDesc));
-  const size_t desc_bytes = align256(off_idx + sizeof(uint32_t) * (size_t)(na + nb + nc));
-  const size_t counted = align256(off_idx + 12 * (size_t)P * (size_t)((N + 127) / 128)) - off_idx +
-                         desc_bytes;
+  const size_t desc_bytes = align256(off_pd + sizeof(ProdDesc));
+  const size_t counted = align256(
+      align256(desc_bytes + 12 * (size_t)P * (size_t)((N + 127) / 128)) +
+      sizeof(uint32_t) * (size_t)(na + nb + nc));
   const size_t res_bytes = sizeof(uint32_t) * (size_t)(na + nb + nc) * poly;
   if (counted > kNoAllocDescBytes || counted + res_bytes > kNoAllocScratchBytes)
     return set_error(kErrTooLarge,
@@ -179,7 +179,6 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
   FwdDesc* fwd = reinterpret_cast<FwdDesc*>(hd + off_fwd);
   InvDesc* inv = reinterpret_cast<InvDesc*>(hd + off_inv);
   ProdDesc* pd = reinterpret_cast<ProdDesc*>(hd + off_pd);
-  uint32_t* idx = reinterpret_cast<uint32_t*>(hd + off_idx);
   pd->m = (uint16_t)m;
   pd->k = (uint16_t)k;
   pd->n = (uint16_t)n;
@@ -189,13 +188,19 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
   pd->a_res = 0;
   pd->b_res = (uint64_t)na * poly;
   pd->c_res = (uint64_t)(na + nb) * poly;
+  // the operands are two buffers: limbs are counted from address 0, so that
+  // one launch takes both (each from its own pointer if one is not aligned)
+  const uintptr_t pa = reinterpret_cast<uintptr_t>(d_a_limbs),
+                  pb = reinterpret_cast<uintptr_t>(d_b_limbs);
+  const bool together = ((pa | pb) & 7) == 0;
+  const uint64_t base_a = together ? pa >> 3 : 0, base_b = together ? pb >> 3 : 0;
   for (int64_t i = 0; i < na + nb; ++i) {
     const bool isb = i >= na;
     const int64_t e2 = isb ? i - na : i;
     const int32_t sz = isb ? b_sizes[e2] : a_sizes[e2];
     const int64_t nl = sz < 0 ? -(int64_t)sz : sz;
     FwdDesc& f = fwd[i];
-    f.limb_off = nl ? (uint64_t)(isb ? b_offs[e2] : a_offs[e2]) : 0;
+    f.limb_off = nl ? (isb ? base_b : base_a) + (uint64_t)(isb ? b_offs[e2] : a_offs[e2]) : 0;
     f.res_off = (isb ? pd->b_res : pd->a_res) + (uint64_t)e2 * poly;
     f.size = sz;
     f.r = (uint32_t)r;
@@ -205,7 +210,6 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
     f.ncoef = (uint32_t)(nco < N ? nco : N);
     f.tile_np = 0;  // plain layout (this entry point contracts on CUDA cores)
     f.tile_e = 0;
-    idx[i] = (uint32_t)i;
   }
   const uint64_t ncoef_c = (uint64_t)(prm.lenA + prm.lenB - 1);
   for (int64_t i = 0; i < nc; ++i) {
@@ -218,7 +222,6 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
     d.lgN = (uint16_t)lgN;
     d.P = (uint16_t)P;
     d.entry = (uint32_t)i;
-    idx[na + nb + i] = (uint32_t)i;
   }
   // segments of the results; their records take the place of the operands'
   // residues, which nothing reads after the contraction
@@ -227,11 +230,8 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
                   (uint64_t)(na + nb) * poly / (sizeof(CrtRec) / sizeof(uint32_t)));
   uint8_t* dd = ds->scratch;
   uint32_t* dres = reinterpret_cast<uint32_t*>(ds->scratch + desc_bytes);
-  // every check has passed: only now is anything of the caller's touched.
-  // Results start cleared: every size is rewritten by the CRT kernel or
-  // stays 0.
-  if ((e = cudaMemsetAsync(d_c_sizes, 0, sizeof(int32_t) * (size_t)nc, s)) != cudaSuccess)
-    return cufail(e, "cudaMemsetAsync(sizes)");
+  // every check has passed: only now is anything of the caller's touched
+  // (the CRT writes every result's size)
   // a copy from pageable memory: it returns once the descriptors are staged,
   // so the next call may reuse g_host_desc
   if ((e = cudaMemcpyAsync(dd, hd, desc_bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess)
@@ -239,14 +239,18 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
   const FwdDesc* dfwd = reinterpret_cast<const FwdDesc*>(dd + off_fwd);
   const InvDesc* dinv = reinterpret_cast<const InvDesc*>(dd + off_inv);
   const ProdDesc* dpd = reinterpret_cast<const ProdDesc*>(dd + off_pd);
-  const uint32_t* didx = reinterpret_cast<const uint32_t*>(dd + off_idx);
 
-  if ((e = launch_split_fwd(dfwd, didx, (int)na, P, lgN, d_a_limbs, dres, ds->twf, s)) !=
-          cudaSuccess ||
-      (e = launch_split_fwd(dfwd, didx + na, (int)nb, P, lgN, d_b_limbs, dres, ds->twf, s)) !=
-          cudaSuccess ||
-      (e = launch_contract_one(dpd, *pd, ds->sms, dres, s)) != cudaSuccess ||
-      (e = launch_inv_ntt(dinv, didx + na + nb, (int)nc, P, lgN, dres, ds->twi, s)) !=
+  const int D = (r + 29) / 30;
+  if (together) {
+    e = launch_fwd_uniform(dfwd, (uint32_t)(na + nb), lgN, P, D, ds->sms, nullptr, dres, ds->twf,
+                           s);
+  } else if ((e = launch_fwd_uniform(dfwd, (uint32_t)na, lgN, P, D, ds->sms, d_a_limbs, dres,
+                                     ds->twf, s)) == cudaSuccess) {
+    e = launch_fwd_uniform(dfwd + na, (uint32_t)nb, lgN, P, D, ds->sms, d_b_limbs, dres, ds->twf,
+                           s);
+  }
+  if (e != cudaSuccess || (e = launch_contract_one(dpd, *pd, ds->sms, dres, s)) != cudaSuccess ||
+      (e = launch_inv_uniform(dinv, (uint32_t)nc, lgN, P, ds->sms, dres, ds->twi, s)) !=
           cudaSuccess ||
       (e = launch_crt_uniform(dinv, (int)nc, crt, P, r, dres,
                               reinterpret_cast<uint32_t*>(d_c_limbs), d_c_sizes,
