@@ -1113,56 +1113,50 @@ constexpr int kCrtWarps = 4;       // entries per CTA
 constexpr int kCrtSteps = 8;       // 32-word steps per tile
 constexpr int kCrtTileWords = 32 * kCrtSteps;
 constexpr size_t kCrtSmemLimit = 200 * 1024;
+// scratch words of a coefficient: P + 1 of them used, an odd number apart
+// (the lanes' stores spread over the banks)
+template <int P>
+constexpr int kCrtStride = (P + 1) | 1;
 
 // Explicit CRT of one coefficient (constants in CrtConst): the symmetric
 // residue X in (-M_P/4, M_P/4) as P words of two's complement.
 template <int P>
-__device__ __forceinline__ void crt_coeff(const uint32_t* __restrict__ res, uint64_t res_off,
-                                          int lgN, int64_t ic, uint32_t (&X)[P]) {
-  const uint64_t N = (uint64_t)1 << lgN;
-  uint32_t y[P];
+__device__ __forceinline__ void crt_coeff(const uint32_t* __restrict__ src, uint32_t N, int lgN,
+                                          uint32_t (&X)[P]) {
+  int32_t y[P];
   uint64_t frac = 0;
 #pragma unroll
   for (int j = 0; j < P; ++j) {
     const uint32_t p = c_primes[j].p;
-    const uint32_t x = __ldg(res + res_off + (uint64_t)j * N + (uint64_t)ic);  // [0, 2p)
-    y[j] = redc((uint64_t)x * c_crt.cm[P][lgN][j], p, c_primes[j].pinv);
-    frac += (uint64_t)y[j] * c_crt.fq[j];
+    const uint64_t T = (uint64_t)__ldg(src) * c_crt.cm[P][lgN][j];  // [0, 2p) times [0, p)
+    src += N;
+    const uint32_t m = (uint32_t)T * c_primes[j].pinv;
+    uint32_t v = (uint32_t)((T + (uint64_t)m * p) >> 32);  // [0, 2p)
+    // beyond eight primes the columns below have room for [0, p) only
+    if (P > 8) v = min(v, v - p);
+    y[j] = (int32_t)v;
+    frac += (uint64_t)v * c_crt.fq[j];
   }
-  const uint32_t q = (uint32_t)((frac + (1ull << 57)) >> 58);  // nearest integer
-  // sum_j y_j (M_P / p_j) in base-2^30 columns (M_P / p_j has P - 1 digits):
-  // products below 2^60, at most 16 per column, no carries inside the sum
-  uint64_t acc[P];
+  const int32_t q = (int32_t)((frac + (1ull << 57)) >> 58);  // nearest integer
+  // sum_j y_j (M_P / p_j) - q M_P in balanced base-2^30 columns, no carries
+  // inside the sums
+  int64_t acc[P];
 #pragma unroll
-  for (int w = 0; w < P; ++w) acc[w] = 0;
+  for (int w = 0; w < P; ++w) acc[w] = -(int64_t)q * c_crt.M30[P][w];
 #pragma unroll
   for (int j = 0; j < P; ++j)
 #pragma unroll
-    for (int w = 0; w + 1 < P; ++w) acc[w] += (uint64_t)y[j] * c_crt.mop30[P][j][w];
-  // digits: carry-normalise (column + carry < 2^64), then subtract q M_P with
-  // a signed borrow; the top digit is 0 for X >= 0 and -1 for X < 0
-  uint32_t dg[P];
-  uint64_t cy = 0;
-#pragma unroll
-  for (int w = 0; w < P; ++w) {
-    const uint64_t t = acc[w] + cy;
-    dg[w] = (uint32_t)t & 0x3fffffffu;
-    cy = t >> 30;
-  }
-  int64_t b = 0;
-#pragma unroll
-  for (int w = 0; w < P; ++w) {
-    const int64_t e = (int64_t)dg[w] - (int64_t)q * (int64_t)c_crt.M30[P][w] + b;
-    dg[w] = (uint32_t)e & 0x3fffffffu;
-    b = e >> 30;  // arithmetic: floor division
-  }
-  const bool neg = ((int64_t)cy + b) < 0;
-  // repack the 30P bits to P 32-bit words of the two's complement value
+    for (int w = 0; w < P; ++w) acc[w] += (int64_t)y[j] * c_crt.mop30[P][j][w];
+  // one signed carry pass to digits in [0, 2^30); what is left over is 0 for
+  // X >= 0 and -1 for X < 0.  The 30P bits go to P 32-bit words on the way.
+  int64_t cy = 0;
   uint64_t buf = 0;
   int bits = 0, wi = 0;
 #pragma unroll
   for (int w = 0; w < P; ++w) {
-    buf |= (uint64_t)dg[w] << bits;
+    const int64_t t = acc[w] + cy;
+    buf |= (uint64_t)((uint32_t)t & 0x3fffffffu) << bits;
+    cy = t >> 30;  // arithmetic: floor division
     bits += 30;
     if (bits >= 32) {
       X[wi++] = (uint32_t)buf;
@@ -1170,7 +1164,7 @@ __device__ __forceinline__ void crt_coeff(const uint32_t* __restrict__ res, uint
       bits -= 32;
     }
   }
-  const uint32_t fill = neg ? 0xffffffffu : 0u;
+  const uint32_t fill = cy < 0 ? 0xffffffffu : 0u;
 #pragma unroll
   for (int w = 0; w < P; ++w) {
     if (w < wi) continue;
@@ -1244,7 +1238,11 @@ __device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* __re
   // so index arithmetic is 32-bit and the divisions by r are multiply-highs
   const int r = (int)d.r;
   const FastDiv divr((uint32_t)r);
+  const uint32_t half_r = 0x80000000u / (uint32_t)r;  // see the division by r below
+  const int reach = (32 * P + 31) / r + 1;  // most coefficients that meet in a word
   const int ncoef = (int)d.ncoef;
+  const uint32_t* __restrict__ src = res + d.res_off;
+  const uint32_t N = 1u << d.lgN;
   uint32_t* o = out + d.out_word;
 
   int hi_prev = 0, carry = 0;
@@ -1263,21 +1261,20 @@ __device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* __re
     // coefficient i = lo_i + c as X_i 2^(i r mod 32): P + 1 words, the top
     // one signed (it carries the sign's borrow), so output word w adds word
     // w - floor(i r / 32) of every coefficient that reaches it
+#pragma unroll 1
     for (int c = lane; c < ncf; c += 32) {
       uint32_t X[P];
-      crt_coeff<P>(res, d.res_off, d.lgN, lo_i + c, X);
+      crt_coeff<P>(src + lo_i + c, N, d.lgN, X);
       const uint32_t sh = (uint32_t)((lo_i + c) * r) & 31u;
-      uint32_t* v = sV + c * (P + 1);
-      uint32_t prev = 0;
+      uint32_t* v = sV + c * kCrtStride<P>;
+      v[0] = X[0] << sh;
 #pragma unroll
-      for (int q = 0; q < P; ++q) {
-        v[q] = sh ? ((X[q] << sh) | (prev >> (32u - sh))) : X[q];
-        prev = X[q];
-      }
-      const uint32_t fill = (uint32_t)((int32_t)X[P - 1] >> 31);
-      v[P] = sh ? ((fill << sh) | (prev >> (32u - sh))) : fill;
+      for (int q = 1; q < P; ++q) v[q] = __funnelshift_l(X[q - 1], X[q], sh);
+      v[P] = __funnelshift_l(X[P - 1], (uint32_t)((int32_t)X[P - 1] >> 31), sh);
     }
     __syncwarp();
+    const int bit0 = lo_i * r;  // where the tile's first coefficient starts
+#pragma unroll 1
     for (int st = 0; st < kCrtSteps; ++st) {
       const int ws = w0 + 32 * st;
       if (ws >= wt) break;
@@ -1285,18 +1282,27 @@ __device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* __re
       const bool active = w < wend;
       int64_t sw = 0;
       if (active) {
-        int ia = lo_i;
-        if (32 * w > 32 * P) {
-          const int t = (int)divr((uint32_t)(32 * w - 32 * P + r - 1));
-          if (t > ia) ia = t;
-        }
-        int ib = (int)divr((uint32_t)(32 * w + 31));
-        if (ib > hi_i) ib = hi_i;
-        // 0 <= w - floor(i r / 32) <= P for every i in [ia, ib]
-        for (int i = ia; i <= ib; ++i) {
-          const int q = w - ((i * r) >> 5);
-          const uint32_t x = sV[(i - lo_i) * (P + 1) + q];
-          sw += q == P ? (int64_t)(int32_t)x : (int64_t)x;
+        // the last coefficient that reaches word w starts at or before its
+        // top bit x = 32 w + 31 - bit0 (below 2^14): floor(x / r) as the
+        // multiply-high of 2x + 1 by floor(2^31 / r), which errs by less than
+        // 2^-17 below (2x + 1) / (2r), at least 1 / (2r) above an integer
+        int b = 32 * w + 31 - bit0;
+        int c = (int)__umulhi(2u * (uint32_t)b + 1u, half_r);
+        if (c > ncf - 1) c = ncf - 1;
+        b -= c * r;
+        // b: from the coefficient's first bit up to the word's top bit, so
+        // the word takes word b / 32 of it; earlier ones lie r bits further
+        const uint32_t* v = sV + c * kCrtStride<P>;
+#pragma unroll 1
+        for (int t = 0; t < reach; ++t) {
+          const int q = b >> 5;
+          if (c >= 0 && q <= P) {
+            const uint32_t x = v[q];
+            sw += q == P ? (int64_t)(int32_t)x : (int64_t)x;
+          }
+          --c;
+          v -= kCrtStride<P>;
+          b += r;
         }
       }
       const int hi = active ? (int)(sw >> 32) : 0;
@@ -1359,7 +1365,7 @@ __device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* __re
         o[w] = F;
         if (!SEG || !unknown) {
           if (F != 0u) {
-            if (w < first_nz) first_nz = w;
+            first_nz = min(first_nz, w);
             last_nz = w;
           }
           if (F != 0xffffffffu) last_no = w;
@@ -1440,12 +1446,19 @@ __device__ __forceinline__ void crt_dispatch(const InvDesc& d, const CrtItem& it
   }
 }
 
-// Prime counts PLO..PHI in one launch, one warp an item, longest first across
-// the counts (the launch has one tail instead of one per count): segments
-// (SEG; segs, or u where all entries are alike), or whole entries (idx, or
-// entries 0, 1, ...).  Each warp's scratch holds warp_words words.
+// Prime counts PLO..PHI in one launch (one tail instead of one per count), one
+// warp an item: segments (SEG; segs, or u where all entries are alike), or
+// whole entries (idx, or entries 0, 1, ...).  Each warp's scratch holds
+// warp_words words.
+//
+// Bound by integer issue and, over mixed prime counts, by instruction fetch:
+// each count is code of its own, so loops stay rolled and the lists are in
+// prime count order.  64 x 64 entries of 65538 words (10 primes) 3190 us,
+// 3650 with the columns' carries, the subtraction of q M and the repacking in
+// passes of their own and two checked divisions a word; 512 mixed products
+// 1763 us, 1995 before.
 template <int PLO, int PHI, bool SEG>
-__global__ void __launch_bounds__(32 * kCrtWarps)
+__global__ void __launch_bounds__(32 * kCrtWarps, PLO > 2 ? 6 : 7)
 k_crt_mixed(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs,
             const uint32_t* __restrict__ idx, int count, CrtUniform u,
             const uint32_t* __restrict__ res, uint32_t* __restrict__ out,
@@ -2498,10 +2511,10 @@ static int crt_cmax(int P, int rmin) {
 }
 
 // Words a warp takes of an entry when a launch writes total_words words: as
-// many as leave every SM kCrtSegWarps warps (a little over two waves of
-// them, so that no long entry is the launch's tail), in whole tiles less the
-// 32 words of the look below a segment.
-constexpr int kCrtSegWarps = 64;
+// many as leave every SM kCrtSegWarps warps (a few waves of them, so that no
+// long entry is the launch's tail), in whole tiles less the 32 words of the
+// look below a segment.
+constexpr int kCrtSegWarps = 128;
 static int crt_segment_words(uint64_t total_words, int sms) {
   const uint64_t t = total_words / ((uint64_t)(sms > 0 ? sms : 1) * kCrtSegWarps);
   const uint64_t tiles = (t + 32 + kCrtTileWords - 1) / kCrtTileWords;
@@ -2513,10 +2526,11 @@ static int crt_segment_words(uint64_t total_words, int sms) {
 // up to two segments stays whole, and where a warp an entry fills the SMs
 // only entries well above the others are split (4096 entries of 2050 words
 // took 121 us whole, 140 in five segments; 2000 of 630 words 33 and 38; 256
-// mixed products 950 us with the long entries split, 1000 without).
+// mixed products 940 us with the long entries split, 1030 without; 512 of
+// them 1763 whole, 1835 with entries above four segments split).
 constexpr uint32_t kCrtShort = 16 * kCrtTileWords;
 static uint32_t crt_split(uint32_t W, uint32_t seg, bool few, uint32_t* step) {
-  const bool split = few ? W > 2 * seg : W > kCrtShort && W > 3 * seg;
+  const bool split = few ? W > 2 * seg : W > kCrtShort && W > 6 * seg;
   uint32_t ns = split ? (W + seg - 1) / seg : 1u;
   *step = (((W + ns - 1) / ns) + 31) & ~31u;
   return ns > 1 ? (W + *step - 1) / *step : 1u;
@@ -2534,15 +2548,18 @@ CrtUniform crt_uniform(uint32_t words, uint32_t count, int sms, uint64_t max_rec
 
 void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, uint32_t* nrecs,
                std::vector<CrtItem>* segs) {
-  // longest entries first (the warp that gets one works longest), ties in
-  // entry order: one sort of packed (longest-first key, index) integers,
-  // which the entries of a single product need not
+  // by prime count, most first (each count is code of its own, and warps that
+  // run side by side share the instruction cache: 1870 -> 1800 us for the
+  // first 512 products of the default batch), then longest first (the warp
+  // that gets one works longest), ties in entry order: one sort of packed
+  // integers, which the entries of a single product need not
   std::vector<uint64_t> keys(idx->size());
   uint64_t total = 0;
   for (size_t i = 0; i < keys.size(); ++i) {
     const uint32_t W = descs[(*idx)[i]].out_words;
     total += W;
-    keys[i] = ((uint64_t)(0xffffffffu - W) << 32) | (*idx)[i];
+    keys[i] = ((uint64_t)(kMaxPrimes - descs[(*idx)[i]].P) << 59) | ((uint64_t)(0x7ffffffu - W) << 32) |
+              (*idx)[i];
   }
   if (!std::is_sorted(keys.begin(), keys.end())) std::sort(keys.begin(), keys.end());
   const uint32_t seg = (uint32_t)crt_segment_words(total, sms);
@@ -2589,7 +2606,7 @@ cudaError_t launch_crt_mixed(const InvDesc* descs, const CrtItem* segs, int nseg
   const int plo = high ? kCrtMixedSplit + 1 : 2, phi = high ? kMaxPrimes : kCrtMixedSplit;
   int words = 0;
   for (int P = plo; P <= phi; ++P)
-    if (rmin[P] > 0) words = std::max(words, crt_cmax(P, rmin[P]) * (P + 1));
+    if (rmin[P] > 0) words = std::max(words, crt_cmax(P, rmin[P]) * ((P + 1) | 1));
   const auto fn = high ? launch_crt<kCrtMixedSplit + 1, kMaxPrimes> : launch_crt<2, kCrtMixedSplit>;
   return fn(descs, segs, nsegs, idx, count, CrtUniform{}, words, res, out, sizes, recs, st);
 }
@@ -2601,7 +2618,7 @@ cudaError_t launch_crt_uniform(const InvDesc* descs, int count, CrtUniform u, in
   const auto fn = P > kCrtMixedSplit ? launch_crt<kCrtMixedSplit + 1, kMaxPrimes>
                                      : launch_crt<2, kCrtMixedSplit>;
   return fn(descs, nullptr, seg ? count * (int)u.nseg : 0, nullptr, seg ? 0 : count, u,
-            crt_cmax(P, r) * (P + 1), res, out, sizes, recs, st);
+            crt_cmax(P, r) * ((P + 1) | 1), res, out, sizes, recs, st);
 }
 
 // Dynamic shared memory limits of every kernel, set once per device at

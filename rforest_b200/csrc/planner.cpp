@@ -118,6 +118,17 @@ std::vector<uint32_t> to_base30(const std::vector<uint32_t>& w32) {
   return out;
 }
 
+// base-2^30 digits -> `count` digits of which all but the last lie in
+// [-2^29, 2^29)
+void balance30(const std::vector<uint32_t>& digits, int count, int32_t* out) {
+  int64_t carry = 0;
+  for (int w = 0; w < count; ++w) {
+    int64_t d = (w < (int)digits.size() ? (int64_t)digits[w] : 0) + carry;
+    carry = w + 1 < count && d >= (1 << 29) ? 1 : 0;
+    out[w] = (int32_t)(d - (carry << 30));
+  }
+}
+
 Moduli* g_moduli = nullptr;
 std::once_flag g_once;
 
@@ -192,7 +203,7 @@ void build(Moduli& M) {
     M.crt.Mwords[P] = words;
     for (int q = 0; q < words && q < kMaxCrtWords; ++q) M.crt.M[P][q] = acc[q];
     const std::vector<uint32_t> m30 = to_base30(acc);
-    for (int w = 0; w < kMaxPrimes; ++w) M.crt.M30[P][w] = w < (int)m30.size() ? m30[w] : 0u;
+    balance30(m30, P, M.crt.M30[P]);
     int top = 31;
     while (!((acc.back() >> top) & 1u)) --top;
     M.mbits[P] = 32 * (words - 1) + top;  // floor(log2 M)
@@ -210,8 +221,7 @@ void build(Moduli& M) {
         mop_mod = mop_mod * (M.p[a] % pj) % pj;
       }
       const std::vector<uint32_t> m30 = to_base30(mop);
-      for (int w = 0; w < kMaxPrimes; ++w)
-        M.crt.mop30[P][j][w] = w < (int)m30.size() ? m30[w] : 0u;
+      balance30(m30, P, M.crt.mop30[P][j]);
       const uint64_t inv = powmod(mop_mod, pj - 2, pj);
       const uint64_t r32 = (((uint64_t)1) << 32) % pj;
       for (int lg = 0; lg <= kMaxLgN; ++lg) {
