@@ -821,7 +821,11 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     }
   }
   if (out_entry > 0x7fffffffULL) return set_error(kErrTooLarge, "too many output entries");
-  contract_items(pd_.data(), cc_prods, context().num_sms, &items_);
+  // One product alone: its entries are all alike, so its launches need no
+  // lists (a chain step of 64 entries spent 95 us planning and uploading them).
+  const bool one = pd_.size() == 1 && !fixed_b_;
+  one_cc_ = one && !cc_prods.empty();
+  if (!one_cc_) contract_items(pd_.data(), cc_prods, context().num_sms, &items_);
 
   // launch groups and the shared index array
   // Transforms: team-sized classes (lgN >= 3) are merged into one launch per
@@ -840,6 +844,14 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     for (auto& kv : classes) {
       Group& g = kv.second;
       const int D = fwd ? (g.max_r + 29) / 30 : 0;
+      if (one) {  // its descriptors in order: entries 0, 1, ...
+        g.uniform = (uint32_t)g.idx.size();
+        g.idx.clear();
+        g.D = D;
+        g.large = g.lgN > kMaxLgNOneCta;
+        out.push_back(std::move(g));
+        continue;
+      }
       if (g.lgN < 3 || D > 7) {  // (never a blocked-layout group: lgN >= 3, r <= 192)
         out.push_back(std::move(g));  // radix-2 path
         continue;
@@ -902,8 +914,18 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     }
     if (g.idx.empty()) continue;
     g.crt_high = high != 0;
-    // (Grouping by prime count first, for instruction-cache locality,
-    // measured no better: 11.45 against 11.29 ms on the default step.)
+    if (one) {
+      const InvDesc& d0 = inv_[g.idx[0]];
+      g.uniform = (uint32_t)g.idx.size();
+      g.idx.clear();
+      g.crt = crt_uniform(d0.out_words, g.uniform, context().num_sms, 0xffffffffu);
+      if (g.crt.nseg > 1) {
+        n_recs_ = g.crt.nseg * g.uniform;
+        g.seg_items = n_recs_;
+      }
+      rec_groups_.push_back(std::move(g));
+      continue;
+    }
     Group sg;  // entries in segments: launches of their own
     sg.P = g.P;
     sg.crt_high = g.crt_high;
@@ -1226,9 +1248,15 @@ int Plan::launch_all(cudaStream_t st, bool timed) {
     if (!(g.b_only && b_valid_)) fwd_run.push_back(&g);
   int r = fan_out(ws_, st, (int)fwd_run.size(), [&](int i, cudaStream_t s) -> int {
     const Group& g = *fwd_run[i];
-    if (g.large)
-      CU(launch_large_fwd(d_fwd_, d_idx_ + g.idx_off, (int)g.idx.size(), g.lgN, g.P, g.D,
-                          ctx.num_sms, ws_->d_limbs, ws_->d_res, ctx.d_twf, ctx.twist_f, s),
+    const uint32_t* idx = g.uniform ? nullptr : d_idx_ + g.idx_off;
+    const int count = g.uniform ? (int)g.uniform : (int)g.idx.size();
+    if (g.uniform && !g.large)
+      CU(launch_fwd_uniform(d_fwd_, g.uniform, g.lgN, g.P, g.D, ctx.num_sms, ws_->d_limbs,
+                            ws_->d_res, ctx.d_twf, s),
+         "split+forward NTT launch");
+    else if (g.large)
+      CU(launch_large_fwd(d_fwd_, idx, count, g.lgN, g.P, g.D, ctx.num_sms, ws_->d_limbs,
+                          ws_->d_res, ctx.d_twf, ctx.twist_f, s),
          "split+forward NTT launch (four-step)");
     else if (g.batched)
       CU(launch_fwd_items(d_fwd_, d_idx_, d_cta_ + g.item_off, (int)g.items.size(), g.D, g.team,
@@ -1242,6 +1270,8 @@ int Plan::launch_all(cudaStream_t st, bool timed) {
   });
   if (r != kOk) return r;
   if (timed) CU(cudaEventRecord(ev[1], st), "cudaEventRecord");
+  if (one_cc_)
+    CU(launch_contract_one(d_pd_, pd_[0], ctx.num_sms, ws_->d_res, st), "contraction launch");
   if (!items_.empty())
     CU(launch_contract(d_pd_, d_items_, (int)items_.size(), ws_->d_res, st), "contraction launch");
   if (!tc_items_.empty())
@@ -1252,9 +1282,14 @@ int Plan::launch_all(cudaStream_t st, bool timed) {
   if (timed) CU(cudaEventRecord(ev[2], st), "cudaEventRecord");
   r = fan_out(ws_, st, (int)inv_groups_.size(), [&](int i, cudaStream_t s) -> int {
     const Group& g = inv_groups_[i];
-    if (g.large)
-      CU(launch_large_inv(d_inv_, d_idx_ + g.idx_off, (int)g.idx.size(), g.lgN, g.P, ctx.num_sms,
-                          ws_->d_res, ctx.d_twi, ctx.twist_i, s),
+    const uint32_t* idx = g.uniform ? nullptr : d_idx_ + g.idx_off;
+    const int count = g.uniform ? (int)g.uniform : (int)g.idx.size();
+    if (g.uniform && !g.large)
+      CU(launch_inv_uniform(d_inv_, g.uniform, g.lgN, g.P, ctx.num_sms, ws_->d_res, ctx.d_twi, s),
+         "inverse NTT launch");
+    else if (g.large)
+      CU(launch_large_inv(d_inv_, idx, count, g.lgN, g.P, ctx.num_sms, ws_->d_res, ctx.d_twi,
+                          ctx.twist_i, s),
          "inverse NTT launch (four-step)");
     else if (g.batched)
       CU(launch_inv_items(d_inv_, d_idx_, d_cta_ + g.item_off, (int)g.items.size(), g.team,
@@ -1270,6 +1305,12 @@ int Plan::launch_all(cudaStream_t st, bool timed) {
   if (timed) CU(cudaEventRecord(ev[3], st), "cudaEventRecord");
   r = fan_out(ws_, st, (int)rec_groups_.size(), [&](int i, cudaStream_t s) -> int {
     const Group& g = rec_groups_[i];
+    if (g.uniform) {
+      CU(launch_crt_uniform(d_inv_, (int)g.uniform, g.crt, g.P, g.rmin[g.P], ws_->d_res, ws_->d_out,
+                            ws_->d_sizes, reinterpret_cast<CrtRec*>(ws_->d_res + off_rec_), s),
+         "CRT+recompose launch");
+      return kOk;
+    }
     CU(launch_crt_mixed(d_inv_, d_crt_ + g.crt_off, (int)g.seg_items, d_idx_ + g.idx_off,
                         (int)g.idx.size(), g.crt_high, g.rmin.data(), ws_->d_res, ws_->d_out,
                         ws_->d_sizes, reinterpret_cast<CrtRec*>(ws_->d_res + off_rec_), s),
@@ -1308,7 +1349,7 @@ void Plan::stage_launches(int64_t out[kStages]) const {
     return n;
   };
   out[0] = count(fwd_groups_);
-  out[1] = (items_.empty() ? 0 : 1) + (tc_items_.empty() ? 0 : 1);
+  out[1] = (items_.empty() && !one_cc_ ? 0 : 1) + (tc_items_.empty() ? 0 : 1);
   out[2] = count(inv_groups_);
   out[3] = 0;
   for (const Group& g : rec_groups_) out[3] += g.seg_items ? kCrtSegLaunches : 1;

@@ -323,6 +323,9 @@ class Plan {
     bool crt_high = false;
     std::vector<int> rmin;
     uint32_t crt_off = 0, seg_items = 0;  // its segments (crt_items)
+    // a plan of one product: its entries, all alike, launched without lists
+    uint32_t uniform = 0;
+    CrtUniform crt;
   };
 
   std::vector<ProductSpec> prods_;
@@ -337,6 +340,7 @@ class Plan {
   std::vector<uint32_t> idx_all_;
   std::vector<CtaItem> cta_items_;
   std::vector<CrtItem> crt_items_;
+  bool one_cc_ = false;    // one product, contracted on CUDA cores without a list
   uint32_t n_recs_ = 0;    // segment records of the CRT, kept behind the residues
   uint64_t off_rec_ = 0;   // first residue word of them
   std::vector<OutRef> outs_;          // flattened output references

@@ -917,7 +917,7 @@ k_fwd_cols(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx, 
   extern __shared__ uint32_t sm[];
   const int e = blockIdx.x / tiles;
   const int tile = blockIdx.x - e * tiles;
-  const FwdDesc d = descs[idx[e]];
+  const FwdDesc d = descs[idx ? idx[e] : e];
   const int lgN = d.lgN;
   const int lgR = lgN - kLargeLgC;
   const int lgW = kLgColPoints - lgR;
@@ -997,12 +997,12 @@ k_ntt_blocks(const FwdDesc* __restrict__ fdescs, const InvDesc* __restrict__ ide
   uint64_t off;
   int lgN, P;
   if (FWD) {
-    const FwdDesc& d = fdescs[idx[e]];
+    const FwdDesc& d = fdescs[idx ? idx[e] : e];
     off = d.res_off;
     lgN = d.lgN;
     P = d.P;
   } else {
-    const InvDesc& d = idescs[idx[e]];
+    const InvDesc& d = idescs[idx ? idx[e] : e];
     off = d.res_off;
     lgN = d.lgN;
     P = d.P;
@@ -1060,7 +1060,7 @@ k_inv_cols(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx, 
   extern __shared__ uint32_t sm[];
   const int e = blockIdx.x / tiles;
   const int tile = blockIdx.x - e * tiles;
-  const InvDesc d = descs[idx[e]];
+  const InvDesc d = descs[idx ? idx[e] : e];
   const int lgN = d.lgN;
   const int lgR = lgN - kLargeLgC;
   const int lgW = kLgColPoints - lgR;

@@ -48,7 +48,7 @@ int prime_chunks(uint64_t ctas, int P, int sms);
 
 // Transforms of 2^16 .. 2^20 points (four-step: column transforms, twist,
 // block transforms), `count` entries of one length 2^lgN in one group (idx
-// lists their descriptors).  Forward: split of D-digit coefficients + the
+// lists their descriptors; nullptr: 0, 1, ...).  Forward: split of D-digit coefficients + the
 // transform; inverse: the transform back to natural order, ready for the
 // CRT.  Two launches each (P primes, cut into chunks where the CTAs are
 // few).  tt: the twist tables of the direction.
