@@ -533,14 +533,10 @@ struct FirstGroup {
         a[q] = digits_residue<D>(dg[0], j, co.neg);
       }
     }
-    const Tw8 t(tw, 1);
-    if (HZ) {
-      fwd_stage0_upper_zero<3>(a, p);
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) bf_fwd(a[q], a[q + 4], t.w1, p, 2 * p);
-    }
-    fwd8<1>(a, t, p);
+    if (HZ)
+      fwd8_first_half(a, Tw8(tw, 1), p);
+    else
+      fwd8_first(a, Tw8(tw, 1), p);
   }
 };
 
@@ -743,7 +739,7 @@ __device__ __forceinline__ void inv_run(uint32_t* __restrict__ io, bool valid, u
       each_group<LGN, TS>(tt, [&](int g) {
         uint32_t a[8];
         load_group<LGN, 0>(s, g, a);
-        inv8(a, t, p);
+        inv8_first(a, t, p);
         if (valid) {
 #pragma unroll
           for (int q = 0; q < 8; ++q) io[q * S::NG + g] = a[q];
@@ -1024,7 +1020,7 @@ k_ntt_blocks(const FwdDesc* __restrict__ fdescs, const InvDesc* __restrict__ ide
     if (FWD) {
 #pragma unroll
       for (int q = 0; q < 8; ++q) a[q] = io[q * S::NG + tid];
-      fwd8(a, Tw8(tw, 1), p);
+      fwd8_first(a, Tw8(tw, 1), p);
       store_group<lgC, 0>(s, tid, a);
       pass_sync<lgC, 0>();
       fwd_middle<lgC, 3, kBlockThreads>(s, 1, j, tid, tables);
@@ -1039,7 +1035,7 @@ k_ntt_blocks(const FwdDesc* __restrict__ fdescs, const InvDesc* __restrict__ ide
       store_run(s, tid, a);
       inv_middle<lgC, S::LAST - 3, kBlockThreads>(s, j, tid, tables);
       load_group<lgC, 0>(s, tid, a);
-      inv8(a, Tw8(tw, 1), p);
+      inv8_first(a, Tw8(tw, 1), p);
       const uint2* th = tt.hi + (size_t)j * kTwistEntries;
       const uint32_t* tl = tt.lo + (size_t)j * kTwistEntries;
       const uint32_t pinv = c_primes[j].pinv;

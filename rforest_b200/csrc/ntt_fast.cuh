@@ -163,14 +163,11 @@ __device__ __forceinline__ void bf_inv(uint32_t& a, uint32_t& b, uint2 S, uint32
   b = mul_shoup_lazy(X - Y + p2, S.x, S.y, p);
 }
 
-// three forward stages (FIRST = 1: the first one is already done)
-template <int FIRST = 0>
+// three forward stages
 __device__ __forceinline__ void fwd8(uint32_t (&a)[8], const Tw8& t, uint32_t p) {
   const uint32_t p2 = 2 * p;
-  if (FIRST == 0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) bf_fwd(a[q], a[q + 4], t.w1, p, p2);
-  }
+  for (int q = 0; q < 4; ++q) bf_fwd(a[q], a[q + 4], t.w1, p, p2);
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     bf_fwd(a[q], a[q + 2], t.w2[0], p, p2);
@@ -190,6 +187,65 @@ __device__ __forceinline__ void inv8(uint32_t (&a)[8], const Tw8& t, uint32_t p)
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) bf_inv(a[q], a[q + 4], t.w1, p, p2);
+}
+
+// The first pass has one group shape: its twiddles are T[1 .. 7], of which
+// T[1], T[2] and T[4] are 1 (the first block of every stage), so seven of its
+// twelve butterflies need no product -- the forward and inverse multiply pipes
+// are as busy as the issue slots.
+__device__ __forceinline__ void bf_one(uint32_t& a, uint32_t& b, uint32_t p2) {
+  const uint32_t U = reduce_2p(a, p2), V = reduce_2p(b, p2);
+  a = U + V;
+  b = U - V + p2;
+}
+__device__ __forceinline__ void fwd8_first(uint32_t (&a)[8], const Tw8& t, uint32_t p) {
+  const uint32_t p2 = 2 * p;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) bf_one(a[q], a[q + 4], p2);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    bf_one(a[q], a[q + 2], p2);
+    bf_fwd(a[q + 4], a[q + 6], t.w2[1], p, p2);
+  }
+  bf_one(a[0], a[1], p2);
+#pragma unroll
+  for (int q = 1; q < 4; ++q) bf_fwd(a[2 * q], a[2 * q + 1], t.w4[q], p, p2);
+}
+// the same where points 4 .. 7 are zero: stage 0 only copies
+__device__ __forceinline__ void fwd8_first_half(uint32_t (&a)[8], const Tw8& t, uint32_t p) {
+  const uint32_t p2 = 2 * p;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) a[q] = a[q + 4] = reduce_2p(a[q], p2);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {  // both inputs below 2p already
+    const uint32_t U = a[q], V = a[q + 2];
+    a[q] = U + V;
+    a[q + 2] = U - V + p2;
+    const uint32_t W = mul_shoup_lazy(a[q + 6], t.w2[1].x, t.w2[1].y, p);
+    a[q + 6] = a[q + 4] - W + p2;
+    a[q + 4] += W;
+  }
+  bf_one(a[0], a[1], p2);
+#pragma unroll
+  for (int q = 1; q < 4; ++q) bf_fwd(a[2 * q], a[2 * q + 1], t.w4[q], p, p2);
+}
+__device__ __forceinline__ void inv8_first(uint32_t (&a)[8], const Tw8& t, uint32_t p) {
+  const uint32_t p2 = 2 * p;
+  auto one = [p2](uint32_t& x, uint32_t& y) {
+    const uint32_t X = x, Y = y;
+    x = reduce_2p(X + Y, p2);
+    y = reduce_2p(X - Y + p2, p2);
+  };
+  one(a[0], a[1]);
+#pragma unroll
+  for (int q = 1; q < 4; ++q) bf_inv(a[2 * q], a[2 * q + 1], t.w4[q], p, p2);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    one(a[q], a[q + 2]);
+    bf_inv(a[q + 4], a[q + 6], t.w2[1], p, p2);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) one(a[q], a[q + 4]);
 }
 
 // the last pass's LP stages on eight consecutive points 8g ..
