@@ -14,9 +14,9 @@
 // operand: the split is four byte permutes per four residues.  The four
 // planes of row i sit in four adjacent TMEM lanes, so one warp holds them:
 // the epilogue weights a lane's sixteen values by 2^(8(s+t)) mod p in 64
-// bits, adds the four lanes' sums with three shuffles (z < 2^57 for
-// k <= 64) and Montgomery-reduces z, so C carries the same 2^-32 factor as
-// the CUDA-core contraction.  Small products pack two or four frequencies
+// bits (two planes t to a product), adds the four lanes' sums with three
+// shuffles (z < 2^62 for k <= 64) and Montgomery-reduces z, so C carries the
+// same 2^-32 factor as the CUDA-core contraction.  Small products pack two or four frequencies
 // into one MMA (Shape).
 //
 // One CTA of 128, 256 or 512 threads (four, two or one an SM, as TMEM and
@@ -44,7 +44,7 @@
 namespace mpzmm {
 namespace tc {
 
-constexpr int kMaxK = 64;        // k <= 64: K' = k bytes padded to 32, z < 2^57
+constexpr int kMaxK = 64;        // k <= 64: K' = k bytes padded to 32, z < 2^62
 constexpr int kBlock = kTcBlock;  // rows i and columns l of C a work item covers
 constexpr int kMaxN = 1024;      // n, m <= 1024: block indices fit the item's 8-bit fields
 constexpr int kMaxM = 1024;

@@ -1635,6 +1635,161 @@ __device__ __forceinline__ void load_freqs(const uint32_t* __restrict__ blk, uin
   }
 }
 
+// Stages the nf frequencies of a packed product (phi > 1): a warp task is 8
+// rows (i of A, l of B) by 16 terms of a slot; a thread gathers four terms'
+// residues of one row for every frequency and writes their byte planes.
+// Small F keeps TU tasks' loads in flight at once.
+template <int F, int NT>
+__device__ __forceinline__ void tc_stage_packed(const ProdDesc& d, const tc::Shape& sh, int m,
+                                                int n, int i_base, int l_base, uint64_t tile0,
+                                                uint32_t sub0, int nf,
+                                                const uint32_t* __restrict__ res, uint8_t* As,
+                                                uint8_t* Bs) {
+  const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+  const int k = d.k, lgphi = sh.phi == 4 ? 2 : 1;
+  const int kbn = (sh.kq + 15) / 16;
+  const int a_tasks = ((m + 7) / 8) * kbn;
+  const int tasks = a_tasks + ((n + 7) / 8) * kbn;
+  constexpr int TU = F <= 4 ? 2 : 1;
+  constexpr int kWarps = NT / 32;
+  for (int task0 = warp; task0 < tasks; task0 += TU * kWarps) {
+    uint32_t x[TU][4][F];
+    int rr[TU], kq[TU];
+    bool isa[TU];
+#pragma unroll
+    for (int w2 = 0; w2 < TU; ++w2) {
+      const int task = task0 + w2 * kWarps;
+      const bool live = task < tasks;
+      const bool isA = task < a_tasks;
+      const int tt = isA ? task : task - a_tasks;
+      const int rb = tt / kbn;
+      const int kb = tt - rb * kbn;
+      const int kk0 = 16 * kb + 4 * (lane & 3);
+      // lane -> (row i of A or column l of B mod 8, term quad)
+      const int r = 8 * rb + (lane >> 2);
+      rr[w2] = r;
+      kq[w2] = kk0;
+      isa[w2] = isA;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int kk = kk0 + c;
+        const bool ok = live && kk < k && r < (isA ? m : n);
+        const uint64_t poly =
+            ok ? (isA ? (uint64_t)((i_base + r) * k + kk) : (uint64_t)(kk * d.n + l_base + r))
+               : 0;
+        load_freqs<F>(res + (isA ? d.a_res : d.b_res),
+                      isA ? (uint64_t)d.m * k : (uint64_t)k * d.n, poly, tile0, sub0, ok, nf,
+                      x[w2][c]);
+      }
+    }
+#pragma unroll
+    for (int w2 = 0; w2 < TU; ++w2) {
+      if (task0 + w2 * kWarps >= tasks) break;  // uniform over the warp
+      const int r = rr[w2], kk0 = kq[w2];
+      if (kk0 >= sh.kq) continue;  // past the slot (a packed slot of 8 or 24 bytes)
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        if (f >= nf) break;
+        // frequency f: group f / phi, slot f mod phi
+        const int g = f >> lgphi, sl = f - (g << lgphi);
+        uint32_t pl[4];
+        tc::byte_planes(x[w2][0][f], x[w2][1][f], x[w2][2][f], x[w2][3][f], pl);
+        // plane s of row i of A (column l of B): row 4 mp sl + 4 r + s of
+        // A' (4 r + s of B'), bytes sl kq + kk; the store order rotates
+        // with bits 3-4 of the lane so every store covers all 32 banks
+        uint8_t* t = isa[w2] ? As + g * sh.a_bytes : Bs + g * sh.b_bytes;
+        const uint32_t row0 = isa[w2] ? (uint32_t)(4 * sh.mp * sl + 4 * r) : (uint32_t)(4 * r);
+        const uint32_t kb = (uint32_t)(sl * sh.kq + kk0);
+        const int gq = (lane >> 3) & 3;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int tp = (q + gq) & 3;
+          const uint32_t v = tp == 0 ? pl[0] : (tp == 1 ? pl[1] : (tp == 2 ? pl[2] : pl[3]));
+          *reinterpret_cast<uint32_t*>(t + tc::tile_off(row0 + (uint32_t)tp, kb,
+                                                        (uint32_t)sh.kp)) = v;
+        }
+      }
+    }
+  }
+}
+
+// Stages the nf frequencies of a product with one frequency a group (phi =
+// 1): a warp task is the block's rows of A (or columns of B), a lane each, by
+// 16 terms.  The lane's sixteen loads go out together, and of every
+// frequency it writes four 16-byte rows of a core matrix, plane (q + r / 2)
+// mod 4 in turn q, so that eight lanes' stores cover all banks (rows r and r
+// + 2 lie a multiple of 128 bytes apart).  About 5 instructions a residue;
+// four terms a thread, each plane a 4-byte store at an address of its own,
+// took 67, three quarters of the kernel's: a 64 x 64 x 64 product of 2^20-bit
+// entries contracted in 13.7 ms, in 8.4 now (with the epilogue's weights in
+// pairs; 9.1 without).
+template <int F, int NT>
+__device__ __forceinline__ void tc_stage_rows(const ProdDesc& d, const tc::Shape& sh, int m, int n,
+                                              int i_base, int l_base, uint64_t tile0,
+                                              uint32_t sub0, int nf,
+                                              const uint32_t* __restrict__ res, uint8_t* As,
+                                              uint8_t* Bs) {
+  const int warp = (int)threadIdx.x >> 5, r = (int)threadIdx.x & 31;
+  const int k = d.k;
+  const int chunks = sh.kq / 16;
+  constexpr int FS = F < 4 ? F : 4;  // frequencies in registers at a time
+  for (int task = warp; task < 2 * chunks; task += NT / 32) {
+    const bool isa = task < chunks;
+    const int ch = isa ? task : task - chunks, kk = 16 * ch;
+    if (r >= (isa ? m : n)) continue;  // rows past the block: their results are not read
+    const uint32_t np = (uint32_t)(isa ? d.m * k : k * d.n);
+    const uint32_t step = (isa ? 1u : (uint32_t)d.n) * kTcTile;  // words a term
+    const uint32_t e0 = isa ? (uint32_t)((i_base + r) * k + kk) : (uint32_t)(kk * d.n + l_base + r);
+    const uint32_t* __restrict__ blk = res + (isa ? d.a_res : d.b_res) + (uint64_t)e0 * kTcTile;
+    uint8_t* dst = (isa ? As : Bs) + tc::tile_off(4u * (uint32_t)r, (uint32_t)kk, (uint32_t)sh.kp);
+    const int bytes = isa ? sh.a_bytes : sh.b_bytes;
+#pragma unroll 1
+    for (int fs = 0; fs < F; fs += FS) {
+      const uint32_t h = sub0 + (uint32_t)fs;
+      const uint32_t* __restrict__ src =
+          blk + (tile0 + (h >> kTcTileLg)) * np * (uint64_t)kTcTile + (h & (kTcTile - 1u));
+      uint32_t x[16][FS];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) {
+        const bool ok = kk + t < k;
+        if (FS == 4 && nf == F) {  // h is a multiple of 4
+          const uint4 u = ok ? __ldg(reinterpret_cast<const uint4*>(src + (uint32_t)t * step))
+                             : make_uint4(0u, 0u, 0u, 0u);
+          x[t][0] = u.x;
+          x[t][1 % FS] = u.y;
+          x[t][2 % FS] = u.z;
+          x[t][3 % FS] = u.w;
+        } else {
+#pragma unroll
+          for (int f = 0; f < FS; ++f) {
+            const uint32_t hf = h + (uint32_t)f;
+            x[t][f] = ok && fs + f < nf
+                          ? __ldg(blk + (tile0 + (hf >> kTcTileLg)) * np * (uint64_t)kTcTile +
+                                  (hf & (kTcTile - 1u)) + (uint32_t)t * step)
+                          : 0u;
+          }
+        }
+      }
+#pragma unroll
+      for (int f = 0; f < FS; ++f) {
+        if (fs + f >= nf) break;
+        uint8_t* o = dst + (fs + f) * bytes;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t s = (uint32_t)(q + (r >> 1)) & 3u;
+          const uint32_t sel = s | ((4u + s) << 4);  // byte s of either word
+          uint32_t w[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            w[c] = __byte_perm(__byte_perm(x[4 * c][f], x[4 * c + 1][f], sel),
+                               __byte_perm(x[4 * c + 2][f], x[4 * c + 3][f], sel), 0x5410);
+          *reinterpret_cast<uint4*>(o + 16u * s) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+    }
+  }
+}
+
 // NT threads: 128 where four CTAs share an SM (one warp a TMEM lane
 // quadrant), 256 where two do, 512 where one CTA has it to itself.
 template <int F, int NT>
@@ -1659,7 +1814,6 @@ k_contract_tc(const ProdDesc* __restrict__ prods, const TcItem* __restrict__ ite
   const int j = it.prime;
   const uint32_t p = c_primes[j].p;
   const uint32_t pinv = c_primes[j].pinv;
-  const uint32_t mu = c_primes[j].mu;
   const uint64_t stride = (uint64_t)d.P * (uint64_t)N;
   const tc::Shape sh = tc::shape_of(m, k, n, F);
   const int phi = sh.phi;
@@ -1675,11 +1829,9 @@ k_contract_tc(const ProdDesc* __restrict__ prods, const TcItem* __restrict__ ite
   // results of the staged frequencies, F + 1 words an output entry (odd
   // stride: the epilogue's scattered stores spread over the banks)
   uint32_t* outs = reinterpret_cast<uint32_t*>(Bs + G * sh.b_bytes);
-  // this lane's byte plane s of A (rows 4 i + s) and its four weights
-  // 2^(8(s+t)) mod p, t = 0..3
-  uint32_t wt[4];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) wt[t] = (uint32_t)c_primes[j].w8[(lane & 3) + t];
+  // this lane's byte plane s of A (rows 4 i + s): its weights 2^(8(s+t)) mod p
+  // for planes t = 0 and 2 of B
+  const uint32_t wt01 = c_primes[j].w8[lane & 3], wt23 = c_primes[j].w8[(lane & 3) + 2];
   const uint32_t a_base = tc::smem_u32(As), b_base = tc::smem_u32(Bs);
   const uint32_t barp[2] = {tc::smem_u32(&bars[0]), tc::smem_u32(&bars[1])};
 
@@ -1724,74 +1876,11 @@ k_contract_tc(const ProdDesc* __restrict__ prods, const TcItem* __restrict__ ite
     const uint64_t tile0 = ((uint64_t)j << (d.lgN - kTcTileLg)) + (hs >> kTcTileLg);
     const uint32_t sub0 = hs & (kTcTile - 1u);
 
-    // ---- stage A' and B' of the nf frequencies: a warp task is 8 rows
-    // (i of A, l of B) by 16 terms of a slot; a thread gathers four terms'
-    // residues of one row for every frequency and writes their byte planes.
-    // Small F keeps TU tasks' loads in flight at once.
-    const int kbn = (sh.kq + 15) / 16;
-    const int a_tasks = ((m + 7) / 8) * kbn;
-    const int tasks = a_tasks + ((n + 7) / 8) * kbn;
-    constexpr int TU = F <= 4 ? 2 : 1;
-    constexpr int kWarps = NT / 32;
-    for (int task0 = warp; task0 < tasks; task0 += TU * kWarps) {
-      uint32_t x[TU][4][F];
-      int rr[TU], kq[TU];
-      bool isa[TU];
-#pragma unroll
-      for (int w2 = 0; w2 < TU; ++w2) {
-        const int task = task0 + w2 * kWarps;
-        const bool live = task < tasks;
-        const bool isA = task < a_tasks;
-        const int tt = isA ? task : task - a_tasks;
-        const int rb = tt / kbn;
-        const int kb = tt - rb * kbn;
-        const int kk0 = 16 * kb + 4 * (lane & 3);
-        // lane -> (row i of A or column l of B mod 8, term quad)
-        const int r = 8 * rb + (lane >> 2);
-        rr[w2] = r;
-        kq[w2] = kk0;
-        isa[w2] = isA;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int kk = kk0 + c;
-          const bool ok = live && kk < k && r < (isA ? m : n);
-          const uint64_t poly =
-              ok ? (isA ? (uint64_t)((i_base + r) * k + kk) : (uint64_t)(kk * d.n + l_base + r))
-                 : 0;
-          load_freqs<F>(res + (isA ? d.a_res : d.b_res),
-                        isA ? (uint64_t)d.m * k : (uint64_t)k * d.n, poly, tile0, sub0, ok, nf,
-                        x[w2][c]);
-        }
-      }
-#pragma unroll
-      for (int w2 = 0; w2 < TU; ++w2) {
-        if (task0 + w2 * kWarps >= tasks) break;  // uniform over the warp
-        const int r = rr[w2], kk0 = kq[w2];
-        if (kk0 >= sh.kq) continue;  // past the slot (a packed slot of 8 or 24 bytes)
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-          if (f >= nf) break;
-          // frequency f: group f / phi, slot f mod phi
-          const int g = f / phi, sl = f - g * phi;
-          uint32_t pl[4];
-          tc::byte_planes(x[w2][0][f], x[w2][1][f], x[w2][2][f], x[w2][3][f], pl);
-          // plane s of row i of A (column l of B): row 4 mp sl + 4 r + s of
-          // A' (4 r + s of B'), bytes sl kq + kk; the store order rotates
-          // with bits 3-4 of the lane so every store covers all 32 banks
-          uint8_t* t = isa[w2] ? As + g * sh.a_bytes : Bs + g * sh.b_bytes;
-          const uint32_t row0 = isa[w2] ? (uint32_t)(4 * sh.mp * sl + 4 * r) : (uint32_t)(4 * r);
-          const uint32_t kb = (uint32_t)(sl * sh.kq + kk0);
-          const int gq = (lane >> 3) & 3;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int tp = (q + gq) & 3;
-            const uint32_t v = tp == 0 ? pl[0] : (tp == 1 ? pl[1] : (tp == 2 ? pl[2] : pl[3]));
-            *reinterpret_cast<uint32_t*>(t + tc::tile_off(row0 + (uint32_t)tp, kb,
-                                                          (uint32_t)sh.kp)) = v;
-          }
-        }
-      }
-    }
+    // ---- stage A' and B' of the nf frequencies ----
+    if (phi == 1)
+      tc_stage_rows<F, NT>(d, sh, m, n, i_base, l_base, tile0, sub0, nf, res, As, Bs);
+    else
+      tc_stage_packed<F, NT>(d, sh, m, n, i_base, l_base, tile0, sub0, nf, res, As, Bs);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
 
@@ -1860,12 +1949,17 @@ k_contract_tc(const ProdDesc* __restrict__ prods, const TcItem* __restrict__ ite
       const uint32_t laddr = tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(buf * bufcols);
       // the warps of quadrant qd share its (group, M tile, 16-column chunk)
       // items; rows i of the quadrant in tile q: ib0 + 32 q + lane / 4
-      const int per_g = sh.mt * nch;
-      for (int xi = warp >> 2; xi < ngu * per_g; xi += NT / 128) {
-        const int gi = xi / per_g;
-        const int rem = xi - gi * per_g;
-        const int q = rem / nch;
-        const int ch = rem - q * nch;
+      int gi = 0, q = 0, ch = warp >> 2;
+      auto carry = [&] {
+        while (ch >= nch) {
+          ch -= nch;
+          if (++q == sh.mt) {
+            q = 0;
+            ++gi;
+          }
+        }
+      };
+      for (carry(); gi < ngu; ch += NT / 128, carry()) {
         const int f = (g0 + gi) * phi + fl;  // phi = 1 when nunits > 1
         const int ib = ib0 + 32 * q;
         if (fl >= phi || f >= nf || ib >= m) continue;  // warp-uniform: no row here
@@ -1875,10 +1969,10 @@ k_contract_tc(const ProdDesc* __restrict__ prods, const TcItem* __restrict__ ite
         uint64_t part[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint64_t z = 0;
-#pragma unroll
-          for (int t = 0; t < 4; ++t) z += (uint64_t)v[4 * c + t] * wt[t];
-          part[c] = z;
+          // planes t in pairs: v < 2^22 (k <= 64), so v_t + 2^8 v_t+1 fits 32 bits
+          const uint32_t t01 = v[4 * c] + (v[4 * c + 1] << 8);
+          const uint32_t t23 = v[4 * c + 2] + (v[4 * c + 3] << 8);
+          part[c] = (uint64_t)t01 * wt01 + (uint64_t)t23 * wt23;
         }
         // add over the four lanes of row i (planes s), lane s ending with
         // output c = s: swap halves across lane bit 1, then across bit 0
@@ -1890,7 +1984,12 @@ k_contract_tc(const ProdDesc* __restrict__ prods, const TcItem* __restrict__ ite
         z += __shfl_xor_sync(0xffffffffu, h0 ? k0 : k1, 1);
         const int i = ib + (lane >> 2);
         const int l = 4 * ch + (lane & 3);
-        if (i < m && l < nl) outs[(i * n + l0 + l) * (F + 1) + f] = redc64(z, p, pinv, mu);
+        // z 2^-32 mod p in [0, 2p): only the weights 2^32 and 2^40 mod p
+        // reach 30 bits, so z < 2^61 + 2^56 < p 2^32; the inverse transform
+        // takes values below 2p
+        if (i < m && l < nl)
+          outs[(i * n + l0 + l) * (F + 1) + f] =
+              (uint32_t)((z + (uint64_t)((uint32_t)z * pinv) * p) >> 32);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       if (!dbl && u + 1 < U) {  // one buffer: the next MMAs wait for every warp
