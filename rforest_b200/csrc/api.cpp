@@ -2,8 +2,10 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <iterator>
 #include <memory>
 #include <mutex>
+#include <string>
 #include <vector>
 
 #include "../../include/mpzmm_b200.h"
@@ -101,8 +103,32 @@ int mpz_matmul(mpz_t* C, mpz_t* A, int r, mpz_t* B, int d) {
 
 }  // namespace
 
+// A plan of many products with much output runs as up to four parts in turn
+// on the caller's stream, so that the results of one part cross the link
+// while the next parts' kernels run: 256 mixed products (260 MB of results)
+// spent 2.7 ms on kernels and then 4.8 ms on the copy.
 struct mpzmm_plan {
-  Plan plan;
+  std::vector<std::unique_ptr<Plan>> parts;
+  std::vector<size_t> first;  // first product of each part, then the count
+  // several parts: the stream of their result copies, and per part the end of
+  // its kernels and of its copies
+  cudaStream_t copy = nullptr;
+  std::vector<cudaEvent_t> ran, copied;
+  // execute was captured into a caller's graph: its replays record no events
+  // here, so the copies stay on the caller's stream
+  bool captured = false;
+
+  ~mpzmm_plan() {
+    for (auto* v : {&ran, &copied})
+      for (cudaEvent_t e : *v) cudaEventDestroy(e);
+    if (copy) cudaStreamDestroy(copy);
+  }
+  template <class F>
+  int each(F f) {  // the first error ends it
+    for (auto& p : parts)
+      if (const int st = f(*p)) return st;
+    return kOk;
+  }
 };
 
 extern "C" {
@@ -463,6 +489,31 @@ int mpzmm_chain(int count, const mpzmm_matrix* mats, uint64_t* c_limbs, const in
   return run_chain(std::move(steps), pick_stream(stream));
 }
 
+// Products at which the parts of a plan start, then their count: up to four
+// of at least 16 MB of results each (about 300 us on the link, well above a
+// part's launches).
+static std::vector<size_t> plan_parts(const std::vector<ProductSpec>& specs) {
+  constexpr uint64_t kPartLimbs = (16ull << 20) / 8;
+  std::vector<uint64_t> out(specs.size());
+  uint64_t total = 0;
+  for (size_t t = 0; t < specs.size(); ++t) {
+    uint64_t a = 0, b = 0;
+    for (const auto& e : specs[t].a) a = std::max<uint64_t>(a, (uint64_t)std::llabs((long long)e.size));
+    for (const auto& e : specs[t].b) b = std::max<uint64_t>(b, (uint64_t)std::llabs((long long)e.size));
+    out[t] = (a + b) * specs[t].c.size();
+    total += out[t];
+  }
+  const uint64_t n = std::min<uint64_t>({4, total / kPartLimbs, (uint64_t)specs.size()});
+  std::vector<size_t> first{0};
+  uint64_t acc = 0;
+  for (size_t t = 0; t + 1 < specs.size() && first.size() < n; ++t) {
+    acc += out[t];
+    if (acc * n >= total * first.size()) first.push_back(t + 1);
+  }
+  first.push_back(specs.size());
+  return first;
+}
+
 static int plan_create(mpzmm_plan** plan, int count, const mpzmm_product* products,
                        bool fixed_b, void* stream) {
   if (!plan) return set_error(kErrArg, "null plan pointer");
@@ -473,9 +524,29 @@ static int plan_create(mpzmm_plan** plan, int count, const mpzmm_product* produc
   std::vector<ProductSpec> specs;
   if ((st = build_specs_packed(count, products, &specs))) return st;
   std::unique_ptr<mpzmm_plan> p(new mpzmm_plan);
-  p->plan.set_fixed_b(fixed_b);
-  if ((st = p->plan.build(std::move(specs)))) return st;
-  if ((st = p->plan.upload(pick_stream(stream)))) return st;
+  p->first = plan_parts(specs);
+  const size_t n = p->first.size() - 1;
+  size_t outputs = 0;
+  for (size_t i = 0; i < n; ++i) {
+    std::vector<ProductSpec> part(std::make_move_iterator(specs.begin() + (long)p->first[i]),
+                                  std::make_move_iterator(specs.begin() + (long)p->first[i + 1]));
+    p->parts.emplace_back(new Plan);
+    p->parts.back()->set_fixed_b(fixed_b);
+    p->parts.back()->set_first_output(outputs);
+    for (const auto& ps : part) outputs += ps.c.size();
+    if ((st = p->parts.back()->build(std::move(part)))) return st;
+    if ((st = p->parts.back()->upload(pick_stream(stream)))) return st;
+  }
+  if (n > 1) {
+    p->ran.resize(n);
+    p->copied.resize(n);
+    cudaError_t e = cudaStreamCreateWithFlags(&p->copy, cudaStreamNonBlocking);
+    for (auto* v : {&p->ran, &p->copied})
+      for (cudaEvent_t& ev : *v)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e != cudaSuccess)
+      return set_error(kErrCuda, std::string("plan streams: ") + cudaGetErrorString(e));
+  }
   *plan = p.release();
   return kOk;
 }
@@ -492,49 +563,99 @@ int mpzmm_plan_create_fixed_b(mpzmm_plan** plan, int count, const mpzmm_product*
 
 int mpzmm_plan_upload_a(mpzmm_plan* plan, void* stream) {
   if (!plan) return set_error(kErrArg, "null plan");
-  return plan->plan.upload_a(pick_stream(stream));
+  cudaStream_t s = pick_stream(stream);
+  return plan->each([&](Plan& p) { return p.upload_a(s); });
 }
 
 int mpzmm_plan_execute(mpzmm_plan* plan, void* stream) {
   if (!plan) return set_error(kErrArg, "null plan");
-  return plan->plan.execute(pick_stream(stream));
+  cudaStream_t s = pick_stream(stream);
+  if (plan->parts.size() == 1) return plan->parts[0]->execute(s);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+    plan->captured = true;
+  for (size_t i = 0; i < plan->parts.size(); ++i) {
+    if (const int st = plan->parts[i]->execute(s)) return st;
+    if (plan->captured) continue;
+    const cudaError_t e = cudaEventRecord(plan->ran[i], s);
+    if (e != cudaSuccess)
+      return set_error(kErrCuda, std::string("cudaEventRecord: ") + cudaGetErrorString(e));
+  }
+  return kOk;
 }
 
 int mpzmm_plan_download(mpzmm_plan* plan, void* stream) {
   if (!plan) return set_error(kErrArg, "null plan");
-  return plan->plan.download(pick_stream(stream));
+  cudaStream_t s = pick_stream(stream);
+  const size_t n = plan->parts.size();
+  if (n == 1) return plan->parts[0]->download(s);
+  // each part's copies follow its own kernels on the copy stream; a part is
+  // written to its destinations while the later ones' copies run
+  const bool own = !plan->captured;
+  cudaStream_t cs = own ? plan->copy : s;
+  for (size_t i = 0; i < n; ++i) {
+    cudaError_t e = own ? cudaStreamWaitEvent(cs, plan->ran[i], 0) : cudaSuccess;
+    int st = e == cudaSuccess ? plan->parts[i]->download_enqueue(cs) : kOk;
+    if (!st && e == cudaSuccess) e = cudaEventRecord(plan->copied[i], cs);
+    if (!st && e != cudaSuccess)
+      st = set_error(kErrCuda, std::string("result copies: ") + cudaGetErrorString(e));
+    if (st) {
+      cudaStreamSynchronize(cs);  // nothing writes the caller's arrays any more
+      return st;
+    }
+  }
+  // a capacity error of one part leaves the others' results written
+  int status = kOk;
+  for (size_t i = 0; i < n; ++i) {
+    const int st = plan->parts[i]->download_finish(cs, plan->copied[i]);
+    if (st && !status) status = st;
+  }
+  const cudaError_t e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess && !status)
+    status = set_error(kErrCuda, std::string("kernel execution: ") + cudaGetErrorString(e));
+  return status;
 }
 
 int mpzmm_plan_upload(mpzmm_plan* plan, void* stream) {
   if (!plan) return set_error(kErrArg, "null plan");
-  return plan->plan.upload(pick_stream(stream));
+  cudaStream_t s = pick_stream(stream);
+  return plan->each([&](Plan& p) { return p.upload(s); });
 }
 
 void mpzmm_plan_destroy(mpzmm_plan* plan) { delete plan; }
 
 int mpzmm_plan_set_graph(mpzmm_plan* plan, int enable) {
   if (!plan) return set_error(kErrArg, "null plan");
-  plan->plan.set_graph(enable != 0);
+  for (auto& p : plan->parts) p->set_graph(enable != 0);
   return kOk;
 }
 
 int mpzmm_plan_set_timing(mpzmm_plan* plan, int enable) {
   if (!plan) return set_error(kErrArg, "null plan");
-  plan->plan.set_timing(enable != 0);
+  for (auto& p : plan->parts) p->set_timing(enable != 0);
   return kOk;
 }
 
 int mpzmm_plan_stage_times(mpzmm_plan* plan, float* ms, int64_t* launches,
                            int64_t* executes) {
   if (!plan) return set_error(kErrArg, "null plan");
-  float t[Plan::kStages];
-  int st = plan->plan.stage_times(t, executes);
+  float sum[Plan::kStages] = {};
+  int64_t count[Plan::kStages] = {};
+  const int st = plan->each([&](Plan& p) {
+    float t[Plan::kStages];
+    if (const int r = p.stage_times(t, executes)) return r;
+    int64_t l[Plan::kStages];
+    p.stage_launches(l);
+    for (int s = 0; s < Plan::kStages; ++s) {
+      sum[s] += t[s];
+      count[s] += l[s];
+    }
+    return (int)kOk;
+  });
   if (st) return st;
-  int64_t l[Plan::kStages];
-  plan->plan.stage_launches(l);
   for (int s = 0; s < Plan::kStages; ++s) {
-    if (ms) ms[s] = t[s];
-    if (launches) launches[s] = l[s];
+    if (ms) ms[s] = sum[s];
+    if (launches) launches[s] = count[s];
   }
   return kOk;
 }
@@ -542,14 +663,19 @@ int mpzmm_plan_stage_times(mpzmm_plan* plan, float* ms, int64_t* launches,
 int mpzmm_plan_info(const mpzmm_plan* plan, int64_t* launches, int64_t* bytes, int index,
                     int* P, int* r, int* lgN) {
   if (!plan) return set_error(kErrArg, "null plan");
-  if (launches) *launches = plan->plan.launches_per_execute();
-  if (bytes) *bytes = plan->plan.device_bytes();
-  const auto& prm = plan->plan.params();
-  if (index >= 0 && index < (int)prm.size()) {
-    if (P) *P = prm[index].P;
-    if (r) *r = prm[index].r;
-    if (lgN) *lgN = prm[index].lgN;
+  int64_t l = 0, b = 0;
+  for (size_t i = 0; i < plan->parts.size(); ++i) {
+    const Plan& p = *plan->parts[i];
+    l += p.launches_per_execute();
+    b += p.device_bytes();
+    if (index < (int)plan->first[i] || index >= (int)plan->first[i + 1]) continue;
+    const Params& prm = p.params()[(size_t)index - plan->first[i]];
+    if (P) *P = prm.P;
+    if (r) *r = prm.r;
+    if (lgN) *lgN = prm.lgN;
   }
+  if (launches) *launches = l;
+  if (bytes) *bytes = b;
   return kOk;
 }
 

@@ -1397,7 +1397,7 @@ int Plan::download_finish(cudaStream_t st, cudaEvent_t done) {
       __mpz_struct* z = static_cast<__mpz_struct*>(o.mpz);
       if (z->_mp_alloc < nl) __gmpz_realloc(z, (mp_size_t)nl);  // GMP's allocator
     } else if (nl > o.cap) {
-      status = set_error(kErrCapacity, "output entry " + std::to_string(e) + " needs " +
+      status = set_error(kErrCapacity, "output entry " + std::to_string(first_output_ + e) + " needs " +
                                            std::to_string(nl) + " limbs, capacity " +
                                            std::to_string(o.cap));
       ok[e] = 0;

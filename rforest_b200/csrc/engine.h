@@ -267,6 +267,9 @@ class Plan {
   // their products with the same B need only A's split and transforms.
   // Such a plan takes host operands only and does not capture CUDA graphs.
   void set_fixed_b(bool on) { fixed_b_ = on; }
+  // The plan is a part of a larger batch: its first output entry's number
+  // there, for messages.
+  void set_first_output(size_t n) { first_output_ = n; }
   int upload_a(cudaStream_t st) { return upload_sides(st, true); }
   // Runs split+fwd NTT, contraction, inverse NTT, CRT+recompose.  With
   // graph mode on (and timing off) the launches are captured into a CUDA
@@ -401,6 +404,7 @@ class Plan {
   std::vector<cudaEvent_t> events_;  // kStages + 1 per timed execute
   bool use_graph_ = false;
   bool fixed_b_ = false;
+  size_t first_output_ = 0;
   bool check_bounds_ = false;  // the debug bounds check runs before every execute
   int check_bounds(cudaStream_t st);
   bool b_valid_ = false;  // B's transforms in device memory match its limbs
