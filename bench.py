@@ -278,6 +278,12 @@ def run_reference_arm(args, rank, world):
     if rank != 0:
         return
     import multiprocessing as mp
+    from oracle import oracle as O
+    if not O.reference_available():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's CPU path (oracle/_ref) is not built"}),
+              flush=True)
+        return
     workers = cpu_workers()
     ctx = mp.get_context("spawn")
     sample = args.cpu_sample
@@ -333,7 +339,8 @@ def main():
     import multiprocessing as mp
     cpu_pool = None
     workers = cpu_workers()
-    if rank == 0 and world == 1 and not args.no_cpu:
+    from oracle import oracle as O
+    if rank == 0 and world == 1 and not args.no_cpu and O.reference_available():
         # spawn the CPU pool before the first GPU call
         cpu_pool = mp.get_context("spawn").Pool(workers)
 
@@ -472,11 +479,11 @@ def main():
         names = ["split_fwd_ntt", "contract", "inv_ntt", "crt_recompose"]
         dom = int(np.argmax(stage_ms))
         if dom == 0:
-            alg, t_ms, kern, stage = b1, stage_ms[0], "k_fwd2 (split + forward NTT launches)", "fwd"
+            alg, t_ms, kern, stage = b1, stage_ms[0], "k_fwd_team+k_fwd_cta (split + forward NTT launches)", "fwd"
         elif dom == 1:
             alg, t_ms, kern, stage = b2, stage_ms[1], "k_contract", "contract"
         else:
-            alg, t_ms, kern, stage = (b3, stage_ms[2] + stage_ms[3], "k_inv2+k_crt_mixed",
+            alg, t_ms, kern, stage = (b3, stage_ms[2] + stage_ms[3], "k_inv_team+k_inv_cta+k_crt_mixed",
                                       "inv_crt")
         # DRAM bytes per step of the stage: the committed ncu summary of the
         # same workload (dram__bytes_read.sum + dram__bytes_write.sum per
@@ -486,6 +493,8 @@ def main():
         per_launch_s = (t_ms / 1000.0) / max(1, timed)
         achieved = alg / per_launch_s / 1e9
         cpu = None
+        if cpu_pool is None and not args.no_cpu and world == 1:
+            cpu = {"unavailable": "the reference's CPU path (oracle/_ref) is not built"}
         if cpu_pool is not None:
             rate, used, done = cpu_reference_rate(args.workload, 1, args.cpu_sample, workers,
                                                   cpu_pool, count=args.count)
