@@ -424,7 +424,8 @@ void Workspace::release_device() {
 int Workspace::ensure_side() {
   if (fork_ev) return kOk;
   for (int i = 0; i < kSideStreams; ++i) {
-    CU(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking), "cudaStreamCreate");
+    CU(cudaStreamCreateWithPriority(&side[i], cudaStreamNonBlocking, side_priority),
+       "cudaStreamCreate");
     CU(cudaEventCreateWithFlags(&join_ev[i], cudaEventDisableTiming), "cudaEventCreate");
   }
   CU(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming), "cudaEventCreate");

@@ -108,6 +108,7 @@ struct Workspace {
   // events that fork them off and join them back; created on first use.
   static constexpr int kSideStreams = 2;
   bool fanout = true;  // false: every launch on the plan's own stream
+  int side_priority = 0;
   cudaStream_t side[kSideStreams] = {};
   cudaEvent_t fork_ev = nullptr;
   cudaEvent_t join_ev[kSideStreams] = {};
@@ -270,6 +271,8 @@ class Plan {
   // The plan is a part of a larger batch: its first output entry's number
   // there, for messages.
   void set_first_output(size_t n) { first_output_ = n; }
+  // Priority of the side streams of the plan's own workspace.
+  void set_priority(int priority) { own_.side_priority = priority; }
   int upload_a(cudaStream_t st) { return upload_sides(st, true); }
   // Runs split+fwd NTT, contraction, inverse NTT, CRT+recompose.  With
   // graph mode on (and timing off) the launches are captured into a CUDA
