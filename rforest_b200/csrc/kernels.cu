@@ -45,6 +45,35 @@ __constant__ CrtConst c_crt;
 
 constexpr int kTwStride = 1 << kTwiddleLg;  // twiddle entries per prime
 
+// The stages of a single product follow one another as small grids, so each
+// lets the next one's blocks come up while it runs and waits for its
+// predecessor's results here (no effect unless the launch asks for it:
+// launch_next).  5 x 7 x 3 of 20011 bits on device buffers 31.7 us, 40.2 with
+// each launch after the end of the one in front; a chain of 15 products 3.00
+// ms, 3.10.
+__device__ __forceinline__ void stage_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// A launch that may come up before the kernel in front of it in the stream
+// has ended; the kernel must start with stage_begin().
+template <class... P, class... A>
+static cudaError_t launch_next(void (*kernel)(P...), int grid, int threads, size_t smem,
+                               cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // NTT building blocks (shared memory, radix-2)
 //
@@ -307,6 +336,7 @@ __device__ __forceinline__ void contract_tiles(const ProdDesc& d, const Contract
 __global__ void __launch_bounds__(kContractThreads, 6)
 k_contract(const ProdDesc* __restrict__ prods, const ContractItem* __restrict__ items,
            ContractUniform u, uint32_t* __restrict__ res) {
+  stage_begin();
   ContractItem it;
   if (items) {
     it = items[blockIdx.x];
@@ -591,6 +621,7 @@ __global__ void __launch_bounds__(kFwdThreads, 4)
 k_fwd_team(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
            const CtaItem* __restrict__ items, CtaUniform u, const uint64_t* __restrict__ limbs,
            uint32_t* __restrict__ res, const uint2* __restrict__ twf) {
+  stage_begin();
   __shared__ __align__(16) uint32_t buf[2 * kTeamWords];
   const CtaItem item = cta_item(items, u);
   const int lgN = item.lgN;
@@ -645,6 +676,7 @@ __global__ void __launch_bounds__(cta_threads(LGN), 1024 / cta_threads(LGN))
 k_fwd_cta(const FwdDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
           const CtaItem* __restrict__ items, CtaUniform u, const uint64_t* __restrict__ limbs,
           uint32_t* __restrict__ res, const uint2* __restrict__ twf) {
+  stage_begin();
   extern __shared__ __align__(16) uint32_t sm[];
   using S = NttShape<LGN>;
   constexpr int NT = cta_threads(LGN);
@@ -754,6 +786,7 @@ __global__ void __launch_bounds__(kFwdThreads, 6)
 k_inv_team(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
            const CtaItem* __restrict__ items, CtaUniform u, uint32_t* __restrict__ res,
            const uint2* __restrict__ twi) {
+  stage_begin();
   __shared__ __align__(16) uint32_t buf[2 * kTeamWords];
   const CtaItem item = cta_item(items, u);
   const int lgN = item.lgN;
@@ -777,6 +810,7 @@ __global__ void __launch_bounds__(cta_threads(LGN), 1024 / cta_threads(LGN))
 k_inv_cta(const InvDesc* __restrict__ descs, const uint32_t* __restrict__ idx,
           const CtaItem* __restrict__ items, CtaUniform u, uint32_t* __restrict__ res,
           const uint2* __restrict__ twi) {
+  stage_begin();
   extern __shared__ __align__(16) uint32_t sm[];
   const CtaItem item = cta_item(items, u);
   uint32_t* io = res + descs[idx ? idx[item.first] : item.first].res_off;
@@ -1459,6 +1493,7 @@ k_crt_mixed(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs,
             const uint32_t* __restrict__ idx, int count, CrtUniform u,
             const uint32_t* __restrict__ res, uint32_t* __restrict__ out,
             int32_t* __restrict__ out_sizes, CrtRec* __restrict__ recs, int warp_words) {
+  stage_begin();
   extern __shared__ uint32_t sm[];
   const int warp = threadIdx.x >> 5;
   const int slot = blockIdx.x * kCrtWarps + warp;
@@ -1487,6 +1522,7 @@ __global__ void __launch_bounds__(32 * kCrtWarps)
 k_crt_finish(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs, int count,
              CrtUniform un, const CrtRec* __restrict__ recs, uint32_t* __restrict__ out,
              int32_t* __restrict__ out_sizes) {
+  stage_begin();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int slot = blockIdx.x * kCrtWarps + (threadIdx.x >> 5);
@@ -2265,12 +2301,17 @@ static cudaError_t launch_inv(const InvDesc* descs, const uint32_t* idx, const C
   switch (lgN) {
 #define MPZMM_CASE(L)                                                                      \
   case L:                                                                                  \
+    if (!items)                                                                            \
+      return launch_next(k_inv_cta<L>, nitems, cta_threads(L), inv_cta_bytes(L), st, descs, \
+                         idx, items, u, res, twi);                                         \
     k_inv_cta<L><<<nitems, cta_threads(L), inv_cta_bytes(L), st>>>(descs, idx, items, u, res, \
                                                                    twi);                   \
     break;
     MPZMM_CTA_SIZES(MPZMM_CASE)
 #undef MPZMM_CASE
     default:
+      if (!items)
+        return launch_next(k_inv_team, nitems, kFwdThreads, 0, st, descs, idx, items, u, res, twi);
       k_inv_team<<<nitems, kFwdThreads, 0, st>>>(descs, idx, items, u, res, twi);
   }
   return cudaGetLastError();
@@ -2452,8 +2493,8 @@ cudaError_t launch_contract_one(const ProdDesc* prod, const ProdDesc& d, int sms
   u.tiles = contract_tiles_of(d);
   u.per = std::min(u.tiles, contract_per((uint64_t)u.tiles * u.blocks, sms));
   const uint32_t groups = (u.tiles + u.per - 1) / u.per;
-  k_contract<<<groups * u.blocks, kContractThreads, 0, st>>>(prod, nullptr, u, res);
-  return cudaGetLastError();
+  return launch_next(k_contract, (int)(groups * u.blocks), kContractThreads, 0, st, prod,
+                     (const ContractItem*)nullptr, u, res);
 }
 
 __device__ __forceinline__ bool fwd_in_bounds(const FwdDesc& f, const BoundsCaps& c) {
@@ -2683,6 +2724,16 @@ static cudaError_t launch_crt(const InvDesc* descs, const CrtItem* segs, int nse
   if (smem == 0 || smem > kCrtSmemLimit) return cudaErrorInvalidValue;
   constexpr int NT = 32 * kCrtWarps;
   const int gs = (nsegs + kCrtWarps - 1) / kCrtWarps, gw = (count + kCrtWarps - 1) / kCrtWarps;
+  if (!segs && !idx) {  // entries all alike
+    const CrtItem* no_items = nullptr;
+    if (nsegs == 0)
+      return launch_next(k_crt_mixed<PLO, PHI, false>, gw, NT, smem, st, descs, no_items, idx,
+                         count, u, res, out, sizes, recs, warp_words);
+    const cudaError_t e = launch_next(k_crt_mixed<PLO, PHI, true>, gs, NT, smem, st, descs,
+                                      no_items, idx, nsegs, u, res, out, sizes, recs, warp_words);
+    if (e != cudaSuccess) return e;
+    return launch_next(k_crt_finish, gs, NT, 0, st, descs, no_items, nsegs, u, recs, out, sizes);
+  }
   if (nsegs > 0) {
     k_crt_mixed<PLO, PHI, true><<<gs, NT, smem, st>>>(descs, segs, nullptr, nsegs, u, res, out,
                                                       sizes, recs, warp_words);

@@ -48,3 +48,22 @@ def test_sizes(gpu, m, k, n, bits, shift):
     got = PK.Packed(dc.cpu().numpy().view(np.uint64), co, dsz.cpu().numpy()).to_ints()
     assert got == [sum(A[i * k + q] * B[q * n + j] for q in range(k)) for i in range(m)
                    for j in range(n)]
+
+
+@pytest.mark.parametrize("bits", [900, 30000, 400000, 3000000])
+def test_one_product_plan_replayed(gpu, bits):
+    """The same list-free launches in a plan's CUDA graph (their blocks may come
+    up before the stage in front has ended), replayed back to back."""
+    rng = random.Random(bits)
+    A = [rng.getrandbits(bits) * rng.choice((-1, 1)) for _ in range(4)]
+    B = [rng.getrandbits(bits) for _ in range(4)]
+    want = [sum(A[2 * i + q] * B[2 * q + j] for q in range(2)) for i in range(2)
+            for j in range(2)]
+    plan = api.Plan([(2, 2, 2, PK.from_ints(A), PK.from_ints(B))])
+    plan.set_graph(True)
+    for _ in range(3):
+        for _ in range(5):
+            plan.execute()
+        assert plan.download()[0].to_ints() == want
+        plan.holders[0].cl[...] = 0
+    plan.close()
