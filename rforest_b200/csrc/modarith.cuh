@@ -45,13 +45,6 @@ __device__ __forceinline__ uint32_t mod32(uint32_t x, uint32_t p, uint32_t mu) {
   return r >= p ? r - p : r;
 }
 
-// Any 64-bit T  ->  T 2^-32 mod p (fold the high word below p, then REDC).
-__device__ __forceinline__ uint32_t redc64(uint64_t T, uint32_t p, uint32_t pinv,
-                                           uint32_t mu) {
-  uint32_t hi = mod32((uint32_t)(T >> 32), p, mu);
-  return redc(((uint64_t)hi << 32) | (uint32_t)T, p, pinv);
-}
-
 // Shoup companion floor(w 2^32 / p) computed on the device (w < p).
 __device__ __forceinline__ uint32_t shoup_of(uint32_t w, uint32_t p) {
   return (uint32_t)(((uint64_t)w << 32) / p);

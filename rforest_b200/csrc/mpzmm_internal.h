@@ -33,12 +33,9 @@ constexpr int kMaxCrtWords = kMaxPrimes + 1;  // 32-bit words of a CRT value
 struct PrimeConst {
   uint32_t p;        // the prime
   uint32_t pinv;     // -p^{-1} mod 2^32 (Montgomery)
-  uint32_t r2;       // 2^64 mod p
   uint32_t mu;       // floor(2^32 / p) (Barrett for 32-bit words)
   uint32_t b32;      // 2^32 mod p
   uint32_t b32q;     // Shoup companion of b32
-  uint32_t post;     // unused (the CRT scale 2^32 N^{-1} depends on N)
-  uint32_t pad;
   uint32_t dig[8];   // 2^(30 q + 32) mod p: weights of the 30-bit digits of a
                      // coefficient, with the Montgomery factor folded in
   uint32_t w8[8];    // 2^(8 u) mod p: weights of the byte convolutions (tensor cores)

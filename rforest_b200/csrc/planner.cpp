@@ -154,7 +154,6 @@ void build(Moduli& M) {
     uint32_t inv = p;  // Newton iteration for p^{-1} mod 2^32 (p odd)
     for (int i = 0; i < 5; ++i) inv *= 2 - p * inv;
     pc.pinv = (uint32_t)(0u - inv);
-    pc.r2 = (uint32_t)(((unsigned __int128)1 << 64) % p);
     pc.mu = (uint32_t)((((uint64_t)1) << 32) / p);
     pc.b32 = (uint32_t)((((uint64_t)1) << 32) % p);
     pc.b32q = shoup(pc.b32, p);
