@@ -826,7 +826,7 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
   // lists (a chain step of 64 entries spent 95 us planning and uploading them).
   const bool one = pd_.size() == 1 && !fixed_b_;
   one_cc_ = one && !cc_prods.empty();
-  if (!one_cc_) contract_items(pd_.data(), cc_prods, context().num_sms, &items_);
+  if (!one_cc_) contract_items(pd_.data(), cc_prods, context().num_sms, beside_, &items_);
 
   // launch groups and the shared index array
   // Transforms: team-sized classes (lgN >= 3) are merged into one launch per
@@ -842,6 +842,7 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
       const int64_t G = std::max<int64_t>(1, fwd_team_points() >> kv.second.lgN);
       ctas += (kv.second.idx.size() + G - 1) / G;
     }
+    ctas = (uint64_t)((double)ctas * beside_);
     for (auto& kv : classes) {
       Group& g = kv.second;
       const int D = fwd ? (g.max_r + 29) / 30 : 0;
@@ -932,7 +933,7 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     sg.crt_high = g.crt_high;
     sg.rmin = g.rmin;
     sg.crt_off = (uint32_t)crt_items_.size();
-    crt_items(inv_.data(), &g.idx, context().num_sms, &n_recs_, &crt_items_);
+    crt_items(inv_.data(), &g.idx, context().num_sms, beside_, &n_recs_, &crt_items_);
     sg.seg_items = (uint32_t)crt_items_.size() - sg.crt_off;
     if (sg.seg_items) rec_groups_.push_back(std::move(sg));
     if (!g.idx.empty()) rec_groups_.push_back(std::move(g));
@@ -1623,6 +1624,8 @@ int run_batch(std::vector<ProductSpec> specs, cudaStream_t st) {
   }
 
   const size_t nchunks = bounds.size() - 1;
+  uint64_t all_limbs = 0;
+  for (const uint64_t l : limbs) all_limbs += l;
   ctx.batch_chunks = (int64_t)nchunks;
   int s = ensure_pipeline(ctx);
   if (!s) s = ensure_timeline(ctx, nchunks);
@@ -1736,6 +1739,9 @@ int run_batch(std::vector<ProductSpec> specs, cudaStream_t st) {
     part.reserve(bounds[c + 1] - bounds[c]);
     for (size_t t = bounds[c]; t < bounds[c + 1]; ++t) part.push_back(std::move(specs[t]));
     std::unique_ptr<Plan> np(new Plan);
+    uint64_t mine = 1;
+    for (size_t t = bounds[c]; t < bounds[c + 1]; ++t) mine += limbs[t];
+    np->set_beside((double)all_limbs / (double)mine);
     const int64_t t0 = now_ns();
     int r = np->prepare(std::move(part));
     const int64_t tp = now_ns();

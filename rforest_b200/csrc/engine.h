@@ -271,6 +271,9 @@ class Plan {
   // The plan is a part of a larger batch: its first output entry's number
   // there, for messages.
   void set_first_output(size_t n) { first_output_ = n; }
+  // The plan runs beside others, which hold `times` its work together with
+  // it: its work lists are cut for what the GPU then has to do.
+  void set_beside(double times) { beside_ = times < 1.0 ? 1.0 : times; }
   // Priority of the side streams of the plan's own workspace.
   void set_priority(int priority) { own_.side_priority = priority; }
   int upload_a(cudaStream_t st) { return upload_sides(st, true); }
@@ -408,6 +411,7 @@ class Plan {
   bool use_graph_ = false;
   bool fixed_b_ = false;
   size_t first_output_ = 0;
+  double beside_ = 1.0;
   bool check_bounds_ = false;  // the debug bounds check runs before every execute
   int check_bounds(cudaStream_t st);
   bool b_valid_ = false;  // B's transforms in device memory match its limbs

@@ -2461,20 +2461,20 @@ static uint32_t contract_blocks_of(const ProdDesc& d) {
   return (((uint32_t)d.P << d.lgN) + kContractThreads - 1) / kContractThreads;
 }
 
-// Tiles a CTA takes where a launch has `work` tiles (over all blocks of
-// positions): one while the launch is below four times the CTAs that run
-// at once (six an SM), more as it grows.
+// Tiles a CTA takes where the launches that run beside one another have
+// `work` tiles (over all blocks of positions): one while that is below eight
+// times the CTAs that run at once (six an SM), more as it grows.
 static uint32_t contract_per(uint64_t work, int sms) {
   const uint64_t per = work / ((uint64_t)(sms > 0 ? sms : 1) * 24);
   return per < 1 ? 1u : (uint32_t)std::min<uint64_t>(per, 0xffffffffu);
 }
 
 void contract_items(const ProdDesc* prods, const std::vector<uint32_t>& which, int sms,
-                    std::vector<ContractItem>* items) {
+                    double beside, std::vector<ContractItem>* items) {
   uint64_t work = 0;
   for (const uint32_t q : which)
     work += (uint64_t)contract_tiles_of(prods[q]) * contract_blocks_of(prods[q]);
-  const uint32_t per = contract_per(work, sms);
+  const uint32_t per = contract_per((uint64_t)((double)work * beside), sms);
   for (const uint32_t q : which) {
     const uint32_t tiles = contract_tiles_of(prods[q]), nb = contract_blocks_of(prods[q]);
     // equal groups: no short one at the end
@@ -2664,6 +2664,13 @@ static int crt_segment_words(uint64_t total_words, int sms) {
 // took 121 us whole, 140 in five segments; 2000 of 630 words 33 and 38; 256
 // mixed products 940 us with the long entries split, 1030 without; 512 of
 // them 1763 whole, 1835 with entries above four segments split).
+//
+// Both questions are about what is on the GPU, not about one launch: the
+// chunks of a batch overlap one another, so their entries are counted
+// together.  Asked of each chunk alone, 19 of the 33 launches of 512 mixed
+// products in 17 chunks were few and cut 350,000 segments, whose lists the
+// host built and the link carried: 11 ms of planning and 559.4 MB to the
+// device, against 7 ms and 550.0 MB.
 constexpr uint32_t kCrtShort = 16 * kCrtTileWords;
 static uint32_t crt_split(uint32_t W, uint32_t seg, bool few, uint32_t* step) {
   const bool split = few ? W > 2 * seg : W > kCrtShort && W > 6 * seg;
@@ -2682,8 +2689,8 @@ CrtUniform crt_uniform(uint32_t words, uint32_t count, int sms, uint64_t max_rec
   return u;
 }
 
-void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, uint32_t* nrecs,
-               std::vector<CrtItem>* segs) {
+void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, double beside,
+               uint32_t* nrecs, std::vector<CrtItem>* segs) {
   // by prime count, most first (each count is code of its own, and warps that
   // run side by side share the instruction cache: 1870 -> 1800 us for the
   // first 512 products of the default batch), then longest first (the warp
@@ -2698,8 +2705,8 @@ void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, uint32
               (*idx)[i];
   }
   if (!std::is_sorted(keys.begin(), keys.end())) std::sort(keys.begin(), keys.end());
-  const uint32_t seg = (uint32_t)crt_segment_words(total, sms);
-  const bool few = crt_few(keys.size(), sms);
+  const uint32_t seg = (uint32_t)crt_segment_words((uint64_t)((double)total * beside), sms);
+  const bool few = crt_few((uint64_t)((double)keys.size() * beside), sms);
   idx->clear();
   for (const uint64_t key : keys) {
     const uint32_t e = (uint32_t)key, W = descs[e].out_words;

@@ -63,9 +63,10 @@ constexpr int kLargeLaunches = 2;  // kernel launches per direction of a four-st
 // CUDA-core contraction over `count` work items.
 cudaError_t launch_contract(const ProdDesc* prods, const ContractItem* items, int count,
                             uint32_t* res, cudaStream_t st);
-// The work of the products `which` (indices into prods), appended to items.
+// The work of the products `which` (indices into prods), appended to items;
+// launches that run beside this one make the work `beside` times as much.
 void contract_items(const ProdDesc* prods, const std::vector<uint32_t>& which, int sms,
-                    std::vector<ContractItem>* items);
+                    double beside, std::vector<ContractItem>* items);
 // One product alone (its descriptor on the device and here), without a list.
 cudaError_t launch_contract_one(const ProdDesc* prod, const ProdDesc& d, int sms, uint32_t* res,
                                 cudaStream_t st);
@@ -107,15 +108,16 @@ cudaError_t launch_contract_tc(const ProdDesc* prods, const TcItem* items, int c
 // CRT + recompose + sign.  crt_items takes the output entries idx and leaves
 // in it those that a warp each recomposes whole, longest first; entries so
 // long that one warp each would leave the GPU (of `sms` SMs) idle go to
-// segs, their records numbered from *nrecs (advanced).
+// segs, their records numbered from *nrecs (advanced); launches that run
+// beside this one make its entries `beside` times as many.
 // launch_crt_mixed runs both lists over several prime counts: high = false
 // takes entries with 2..kCrtMixedSplit primes, high = true those with more;
 // rmin[P] is the narrowest coefficient width among the entries with P primes
 // (0: none; it sizes the scratch).  One kernel for the whole entries, two
 // for the segments.
 constexpr int kCrtMixedSplit = 10;
-void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, uint32_t* nrecs,
-               std::vector<CrtItem>* segs);
+void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, double beside,
+               uint32_t* nrecs, std::vector<CrtItem>* segs);
 constexpr int kCrtSegLaunches = 2;
 cudaError_t launch_crt_mixed(const InvDesc* descs, const CrtItem* segs, int nsegs,
                              const uint32_t* idx, int count, bool high, const int* rmin,
