@@ -56,6 +56,15 @@ __device__ __forceinline__ void stage_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A load of what the kernel in front writes, in a kernel that starts with
+// stage_begin(): its grid may live while the writer does, and the read-only
+// path (__ldg, const __restrict__) is defined only for memory that nothing
+// writes as long as the grid lives.  The wait orders ordinary loads.
+template <class T>
+__device__ __forceinline__ T stage_load(const T* p) {
+  return __ldca(p);
+}
+
 // A launch that may come up before the kernel in front of it in the stream
 // has ended; the kernel must start with stage_begin().
 template <class... P, class... A>
@@ -235,8 +244,7 @@ __device__ __forceinline__ uint64_t fold64(uint64_t x, uint32_t b32) {
 // R terms (1 to 4) of a tile, their loads issued together.
 template <int TI, int TJ, int R>
 __device__ __forceinline__ void contract_terms(uint64_t (&acc)[TI][TJ],
-                                               const uint32_t* __restrict__ A,
-                                               const uint32_t* __restrict__ B,
+                                               const uint32_t* A, const uint32_t* B,
                                                const uint32_t (&ao)[TI], const uint32_t (&bo)[TJ],
                                                uint32_t stride, uint32_t bstep, uint32_t b32,
                                                int& room) {
@@ -244,9 +252,9 @@ __device__ __forceinline__ void contract_terms(uint64_t (&acc)[TI][TJ],
 #pragma unroll
   for (int u = 0; u < R; ++u) {
 #pragma unroll
-    for (int x = 0; x < TI; ++x) av[u][x] = __ldg(A + ao[x] + (uint32_t)u * stride);
+    for (int x = 0; x < TI; ++x) av[u][x] = stage_load(A + ao[x] + (uint32_t)u * stride);
 #pragma unroll
-    for (int y = 0; y < TJ; ++y) bv[u][y] = __ldg(B + bo[y] + (uint32_t)u * bstep);
+    for (int y = 0; y < TJ; ++y) bv[u][y] = stage_load(B + bo[y] + (uint32_t)u * bstep);
   }
   if (room < R) {
 #pragma unroll
@@ -272,8 +280,8 @@ __device__ __forceinline__ void contract_tiles(const ProdDesc& d, const Contract
   const uint32_t pinv = c_primes[j].pinv;
   const uint32_t b32 = c_primes[j].b32;
   const uint32_t stride = (uint32_t)d.P << d.lgN;  // words between polynomials
-  const uint32_t* __restrict__ A = res + d.a_res + pos;
-  const uint32_t* __restrict__ B = res + d.b_res + pos;
+  const uint32_t* A = res + d.a_res + pos;
+  const uint32_t* B = res + d.b_res + pos;
   uint32_t* C = res + d.c_res + pos;
   const int m = d.m, k = d.k, n = d.n;
   const uint32_t bstep = (uint32_t)n * stride;
@@ -297,8 +305,8 @@ __device__ __forceinline__ void contract_tiles(const ProdDesc& d, const Contract
 #pragma unroll
       for (int y = 0; y < TJ; ++y) acc[x][y] = 0;
     int room = kContractFirst;
-    const uint32_t* __restrict__ Aq = A;
-    const uint32_t* __restrict__ Bq = B;
+    const uint32_t* Aq = A;
+    const uint32_t* Bq = B;
     for (int q = k; q >= 4; q -= 4) {
       contract_terms<TI, TJ, 4>(acc, Aq, Bq, ao, bo, stride, bstep, b32, room);
       Aq += 4 * (uint64_t)stride;
@@ -1151,14 +1159,14 @@ constexpr int kCrtStride = (P + 1) | 1;
 // Explicit CRT of one coefficient (constants in CrtConst): the symmetric
 // residue X in (-M_P/4, M_P/4) as P words of two's complement.
 template <int P>
-__device__ __forceinline__ void crt_coeff(const uint32_t* __restrict__ src, uint32_t N, int lgN,
+__device__ __forceinline__ void crt_coeff(const uint32_t* src, uint32_t N, int lgN,
                                           uint32_t (&X)[P]) {
   int32_t y[P];
   uint64_t frac = 0;
 #pragma unroll
   for (int j = 0; j < P; ++j) {
     const uint32_t p = c_primes[j].p;
-    const uint64_t T = (uint64_t)__ldg(src) * c_crt.cm[P][lgN][j];  // [0, 2p) times [0, p)
+    const uint64_t T = (uint64_t)stage_load(src) * c_crt.cm[P][lgN][j];  // [0, 2p) times [0, p)
     src += N;
     const uint32_t m = (uint32_t)T * c_primes[j].pinv;
     uint32_t v = (uint32_t)((T + (uint64_t)m * p) >> 32);  // [0, 2p)
@@ -1258,7 +1266,7 @@ __device__ __forceinline__ int lookback_carry(uint32_t y, int g, bool prop, int 
 // kernels on 64.  (Two kernels, because the segment's state costs whole
 // entries 8 registers and a CTA less an SM: 9 % of the stage's time.)
 template <int P, bool SEG>
-__device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* __restrict__ res,
+__device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* res,
                                           uint32_t* __restrict__ out,
                                           int32_t* __restrict__ out_sizes, uint32_t* sV,
                                           int wbeg, int wend, CrtRec* __restrict__ rec,
@@ -1271,7 +1279,7 @@ __device__ __forceinline__ void crt_range(const InvDesc& d, const uint32_t* __re
   const uint32_t half_r = 0x80000000u / (uint32_t)r;  // see the division by r below
   const int reach = (32 * P + 31) / r + 1;  // most coefficients that meet in a word
   const int ncoef = (int)d.ncoef;
-  const uint32_t* __restrict__ src = res + d.res_off;
+  const uint32_t* src = res + d.res_off;
   const uint32_t N = 1u << d.lgN;
   uint32_t* o = out + d.out_word;
 
@@ -1464,8 +1472,7 @@ __device__ __forceinline__ CrtItem uniform_item(const CrtUniform& u, uint32_t sl
 
 template <int P, int PHI, bool SEG>
 __device__ __forceinline__ void crt_dispatch(const InvDesc& d, const CrtItem& it,
-                                             const uint32_t* __restrict__ res,
-                                             uint32_t* __restrict__ out,
+                                             const uint32_t* res, uint32_t* __restrict__ out,
                                              int32_t* __restrict__ out_sizes, uint32_t* sU,
                                              CrtRec* __restrict__ rec, int lane) {
   if (d.P == P) {
@@ -1491,8 +1498,8 @@ template <int PLO, int PHI, bool SEG>
 __global__ void __launch_bounds__(32 * kCrtWarps, PLO > 2 ? 6 : 7)
 k_crt_mixed(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs,
             const uint32_t* __restrict__ idx, int count, CrtUniform u,
-            const uint32_t* __restrict__ res, uint32_t* __restrict__ out,
-            int32_t* __restrict__ out_sizes, CrtRec* __restrict__ recs, int warp_words) {
+            const uint32_t* res, uint32_t* __restrict__ out, int32_t* __restrict__ out_sizes,
+            CrtRec* __restrict__ recs, int warp_words) {
   stage_begin();
   extern __shared__ uint32_t sm[];
   const int warp = threadIdx.x >> 5;
@@ -1520,7 +1527,7 @@ k_crt_mixed(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs,
 // runs over the entry's records once, 32 a step.
 __global__ void __launch_bounds__(32 * kCrtWarps)
 k_crt_finish(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs, int count,
-             CrtUniform un, const CrtRec* __restrict__ recs, uint32_t* __restrict__ out,
+             CrtUniform un, const CrtRec* recs, uint32_t* __restrict__ out,
              int32_t* __restrict__ out_sizes) {
   stage_begin();
   const unsigned FULL = 0xffffffffu;
@@ -1529,37 +1536,38 @@ k_crt_finish(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs
   if (slot >= count) return;  // whole warp
   const CrtItem it = segs ? segs[slot] : uniform_item(un, (uint32_t)slot);
   const InvDesc& d = descs[it.inv];
-  const CrtRec* __restrict__ R = recs + it.rec;
+  const CrtRec* R = recs + it.rec;
   const int s = (int)it.seg, S = (int)it.nseg;
   const CrtRec& me = R[s];
   uint32_t* o = out + d.out_word;
-  const bool open = me.open != 0;
+  const bool open = stage_load(&me.open) != 0;
   int cs = 1;        // the carry into this segment, plus one
   bool negative, below;  // the entry's sign; a nonzero word below this segment
   int top;           // (top segment) last word of the magnitude that is not zero
-  if (!open && !R[S - 1].open && (s == 0 || (!R[s - 1].open && R[s - 1].last_nz[1] >= 0)) &&
-      (s != S - 1 || (me.last_nz[1] >= 0 && me.last_no[1] >= 0))) {
-    negative = R[S - 1].top[1] != 0;
+  if (!open && !stage_load(&R[S - 1].open) &&
+      (s == 0 || (!stage_load(&R[s - 1].open) && stage_load(&R[s - 1].last_nz[1]) >= 0)) &&
+      (s != S - 1 || (stage_load(&me.last_nz[1]) >= 0 && stage_load(&me.last_no[1]) >= 0))) {
+    negative = stage_load(&R[S - 1].top[1]) != 0;
     below = s > 0;
-    top = negative ? me.last_no[1] : me.last_nz[1];
+    top = stage_load(negative ? &me.last_no[1] : &me.last_nz[1]);
   } else {
     int c = 1, zf = 0x7fffffff, zb = 0x7fffffff, lz = -1, lo = -1, neg = 0;
     for (int t0 = 0; t0 < S; t0 += 32) {
       const int t = t0 + lane;
       const bool live = t < S;
-      const uint32_t tf = live ? R[t].tf : kTfIdentity;
+      const uint32_t tf = live ? stage_load(&R[t].tf) : kTfIdentity;
       int mc = 1;
 #pragma unroll
       for (int u = 0; u < 32; ++u) {
         if (lane == u) mc = c;
         c = (int)((__shfl_sync(FULL, tf, u) >> (2 * c)) & 3u);
       }
-      const int fn = live ? R[t].first_nz[mc] : 0x7fffffff;
+      const int fn = live ? stage_load(&R[t].first_nz[mc]) : 0x7fffffff;
       zf = min(zf, __reduce_min_sync(FULL, fn));
       zb = min(zb, __reduce_min_sync(FULL, t < s ? fn : 0x7fffffff));
-      lz = max(lz, __reduce_max_sync(FULL, live ? R[t].last_nz[mc] : -1));
-      lo = max(lo, __reduce_max_sync(FULL, live ? R[t].last_no[mc] : -1));
-      neg |= __reduce_max_sync(FULL, t == S - 1 ? R[t].top[mc] : 0);
+      lz = max(lz, __reduce_max_sync(FULL, live ? stage_load(&R[t].last_nz[mc]) : -1));
+      lo = max(lo, __reduce_max_sync(FULL, live ? stage_load(&R[t].last_no[mc]) : -1));
+      neg |= __reduce_max_sync(FULL, t == S - 1 ? stage_load(&R[t].top[mc]) : 0);
       if (s >= t0 && s < t0 + 32) cs = __shfl_sync(FULL, mc, s - t0);
     }
     negative = neg != 0;
@@ -1579,7 +1587,7 @@ k_crt_finish(const InvDesc* __restrict__ descs, const CrtItem* __restrict__ segs
     }
   }
   if (negative) {
-    const int zf = below ? -1 : me.first_nz[cs];
+    const int zf = below ? -1 : stage_load(&me.first_nz[cs]);
     for (int w = w0 + lane; w < w1; w += 32) {
       const uint32_t F = o[w];
       if (w >= zf) o[w] = w == zf ? 0u - F : ~F;
