@@ -284,9 +284,7 @@ typedef struct mpzmm_plan mpzmm_plan;
 MPZMM_API int mpzmm_plan_create(mpzmm_plan **plan, int count, const mpzmm_product *products,
                       void *stream);
 /* Runs every kernel of the plan on the inputs already resident in device
-   memory; results stay on the device.  Asynchronous on `stream` (a plan with
-   32 MB of results or more runs in parts on streams of its own, forked from
-   `stream` and joined to it). */
+   memory; results stay on the device.  Asynchronous on `stream`. */
 MPZMM_API int mpzmm_plan_execute(mpzmm_plan *plan, void *stream);
 /* Copies the results of the last execute into the products' host outputs
    (c_limbs / c_sizes given at create time), a part's while later parts

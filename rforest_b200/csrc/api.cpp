@@ -106,21 +106,19 @@ int mpz_matmul(mpz_t* C, mpz_t* A, int r, mpz_t* B, int d) {
 // A plan of many products with much output runs as up to four parts, so that
 // the results of one part cross the link while the next parts' kernels run:
 // 256 mixed products (260 MB of results) spent 2.7 ms on kernels and then 4.8
-// ms on the copy.  Each part has a stream of its own, forked from the
-// caller's and joined to it, the earlier the higher its priority: a part
-// fills the SMs that the tails of the earlier ones' launches leave.  1024
-// products of the default batch, execute alone / with download: 10.7 / 20.8 ms
-// so, 11.5 ms in turn on one stream, 10.1 / 27.9 undivided.
+// ms on the copy.  The parts' kernels follow one another on the caller's
+// stream, at its priority: on streams of their own they would need priorities
+// above it to keep their order.  256 and 512 mixed products, execute and
+// download: 5.11 and 9.28 ms so, 5.28 and 9.40 on streams of descending
+// priority, 6.91 and 12.82 on streams of one priority; execute alone pays for
+// the tails of every part's launches (1024 products 11.5 ms, 10.1 undivided).
 struct mpzmm_plan {
   std::vector<std::unique_ptr<Plan>> parts;
   std::vector<size_t> first;  // first product of each part, then the count
   // several parts: the stream of their result copies, and per part the end of
   // its kernels and of its copies
   cudaStream_t copy = nullptr;
-  std::vector<cudaStream_t> run;
-  cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> ran, copied;
-  bool timing = false;  // stage times: the parts in turn, or they would overlap
   // execute was captured into a caller's graph: its replays record no events
   // here, so the copies stay on the caller's stream
   bool captured = false;
@@ -128,8 +126,6 @@ struct mpzmm_plan {
   ~mpzmm_plan() {
     for (auto* v : {&ran, &copied})
       for (cudaEvent_t e : *v) cudaEventDestroy(e);
-    for (cudaStream_t s : run) cudaStreamDestroy(s);
-    if (fork) cudaEventDestroy(fork);
     if (copy) cudaStreamDestroy(copy);
   }
   template <class F>
@@ -536,16 +532,12 @@ static int plan_create(mpzmm_plan** plan, int count, const mpzmm_product* produc
   p->first = plan_parts(specs);
   const size_t n = p->first.size() - 1;
   size_t outputs = 0;
-  int least = 0, greatest = 0;
-  if (n > 1) cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  auto priority = [&](size_t i) { return std::min(least, greatest + (int)i); };
   for (size_t i = 0; i < n; ++i) {
     std::vector<ProductSpec> part(std::make_move_iterator(specs.begin() + (long)p->first[i]),
                                   std::make_move_iterator(specs.begin() + (long)p->first[i + 1]));
     p->parts.emplace_back(new Plan);
     p->parts.back()->set_fixed_b(fixed_b);
     p->parts.back()->set_first_output(outputs);
-    p->parts.back()->set_priority(priority(i));
     for (const auto& ps : part) outputs += ps.c.size();
     if ((st = p->parts.back()->build(std::move(part)))) return st;
     if ((st = p->parts.back()->upload(pick_stream(stream)))) return st;
@@ -553,12 +545,7 @@ static int plan_create(mpzmm_plan** plan, int count, const mpzmm_product* produc
   if (n > 1) {
     p->ran.resize(n);
     p->copied.resize(n);
-    p->run.resize(n);
     cudaError_t e = cudaStreamCreateWithFlags(&p->copy, cudaStreamNonBlocking);
-    for (size_t i = 0; i < n; ++i)
-      if (e == cudaSuccess)
-        e = cudaStreamCreateWithPriority(&p->run[i], cudaStreamNonBlocking, priority(i));
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);
     for (auto* v : {&p->ran, &p->copied})
       for (cudaEvent_t& ev : *v)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
@@ -592,28 +579,13 @@ int mpzmm_plan_execute(mpzmm_plan* plan, void* stream) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
     plan->captured = true;
-  // forked from the caller's stream (also inside a capture) and joined to it
-  auto cu = [](cudaError_t e) {
-    return e == cudaSuccess
-               ? (int)kOk
-               : set_error(kErrCuda, std::string("plan parts: ") + cudaGetErrorString(e));
-  };
-  const size_t n = plan->parts.size();
-  int st = cu(cudaEventRecord(plan->fork, s));
-  size_t forked = 0;
-  for (size_t i = 0; i < n && !st; ++i) {
-    cudaStream_t ps = plan->timing ? s : plan->run[i];
-    if (ps != s) st = cu(cudaStreamWaitEvent(ps, plan->fork, 0));
-    if (!st) forked = i + 1;
-    if (!st) st = plan->parts[i]->execute(ps);
-    if (!st) st = cu(cudaEventRecord(plan->ran[i], ps));
+  for (size_t i = 0; i < plan->parts.size(); ++i) {
+    if (const int st = plan->parts[i]->execute(s)) return st;
+    const cudaError_t e = cudaEventRecord(plan->ran[i], s);
+    if (e != cudaSuccess)
+      return set_error(kErrCuda, std::string("plan parts: ") + cudaGetErrorString(e));
   }
-  for (size_t i = 0; i < forked && !plan->timing; ++i) {
-    if (st) cudaEventRecord(plan->ran[i], plan->run[i]);  // join what was launched all the same
-    const cudaError_t e = cudaStreamWaitEvent(s, plan->ran[i], 0);
-    if (!st) st = cu(e);
-  }
-  return st;
+  return kOk;
 }
 
 int mpzmm_plan_download(mpzmm_plan* plan, void* stream) {
@@ -664,7 +636,6 @@ int mpzmm_plan_set_graph(mpzmm_plan* plan, int enable) {
 
 int mpzmm_plan_set_timing(mpzmm_plan* plan, int enable) {
   if (!plan) return set_error(kErrArg, "null plan");
-  plan->timing = enable != 0;
   for (auto& p : plan->parts) p->set_timing(enable != 0);
   return kOk;
 }

@@ -424,8 +424,7 @@ void Workspace::release_device() {
 int Workspace::ensure_side() {
   if (fork_ev) return kOk;
   for (int i = 0; i < kSideStreams; ++i) {
-    CU(cudaStreamCreateWithPriority(&side[i], cudaStreamNonBlocking, side_priority),
-       "cudaStreamCreate");
+    CU(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking), "cudaStreamCreate");
     CU(cudaEventCreateWithFlags(&join_ev[i], cudaEventDisableTiming), "cudaEventCreate");
   }
   CU(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming), "cudaEventCreate");

@@ -108,7 +108,6 @@ struct Workspace {
   // events that fork them off and join them back; created on first use.
   static constexpr int kSideStreams = 2;
   bool fanout = true;  // false: every launch on the plan's own stream
-  int side_priority = 0;
   cudaStream_t side[kSideStreams] = {};
   cudaEvent_t fork_ev = nullptr;
   cudaEvent_t join_ev[kSideStreams] = {};
@@ -274,8 +273,6 @@ class Plan {
   // The plan runs beside others, which hold `times` its work together with
   // it: its work lists are cut for what the GPU then has to do.
   void set_beside(double times) { beside_ = times < 1.0 ? 1.0 : times; }
-  // Priority of the side streams of the plan's own workspace.
-  void set_priority(int priority) { own_.side_priority = priority; }
   int upload_a(cudaStream_t st) { return upload_sides(st, true); }
   // Runs split+fwd NTT, contraction, inverse NTT, CRT+recompose.  With
   // graph mode on (and timing off) the launches are captured into a CUDA
