@@ -489,7 +489,18 @@ int64_t estimate_device_bytes(const ProductSpec& ps, int64_t* host_bytes) {
   const int64_t entries = (int64_t)ps.m * ps.k + (int64_t)ps.k * ps.n + (int64_t)ps.m * ps.n;
   const int64_t res = prm.P ? entries * prm.P * ((int64_t)1 << prm.lgN) * 4 : 0;
   const int64_t out = (int64_t)ps.m * ps.n * prm.out_limbs * 8;
-  const int64_t desc = entries * 64 + 4096;
+  // descriptors, index lists and sizes; segment records and cut work lists
+  int64_t desc = entries * 64 + 4096;
+  if (prm.P) {
+    ProdDesc d{};
+    d.m = (uint16_t)ps.m;
+    d.k = (uint16_t)ps.k;
+    d.n = (uint16_t)ps.n;
+    d.lgN = (uint16_t)prm.lgN;
+    d.P = (uint16_t)prm.P;
+    d.pad = (uint16_t)contract_tile(ps.m, ps.n);
+    desc += cut_list_bytes(d, (uint32_t)(2 * prm.out_limbs), context().num_sms);
+  }
   if (host_bytes) *host_bytes = limbs * 8 + out;
   return limbs * 8 + res + out + desc;
 }

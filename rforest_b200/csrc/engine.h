@@ -127,9 +127,10 @@ struct Workspace {
   ~Workspace() { release(); }
 };
 
-// Device bytes a batch of products will reserve (parameters, residues,
-// limbs, outputs and descriptors), without building it; host_bytes (if
-// given) receives the bytes its inputs and outputs move across the link.
+// Device bytes a product takes in a batch (residues, limbs, outputs,
+// descriptors, segment records and work lists), without building it;
+// host_bytes (if given) receives the bytes its inputs and outputs move across
+// the link.
 int64_t estimate_device_bytes(const ProductSpec& ps, int64_t* host_bytes = nullptr);
 
 // Process-wide device state: tables on the device, default stream.

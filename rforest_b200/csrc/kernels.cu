@@ -2730,6 +2730,34 @@ void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, double
   }
 }
 
+// The product alone: every list is cut finest there, since each rule takes
+// larger pieces as the launches' work grows.
+int64_t cut_list_bytes(const ProdDesc& d, uint32_t words, int sms) {
+  const int64_t entries = (int64_t)d.m * d.n, operands = (int64_t)(d.m + d.n) * d.k;
+  uint32_t step;
+  const uint32_t ns =
+      crt_split(words, (uint32_t)crt_segment_words((uint64_t)words * entries, sms),
+                crt_few((uint64_t)entries, sms), &step);
+  int64_t bytes = ns > 1 ? entries * ns * (int64_t)(sizeof(CrtRec) + sizeof(CrtItem)) : 0;
+  const uint32_t tiles = contract_tiles_of(d), nb = contract_blocks_of(d);
+  const uint32_t per = contract_per((uint64_t)tiles * nb, sms);
+  int64_t contract = (int64_t)((tiles + per - 1) / per) * nb * (int64_t)sizeof(ContractItem);
+  if (contract_tc_eligible(d.m, d.k, d.n)) {
+    const int64_t blocks = (int64_t)((d.m + tc::kBlock - 1) / tc::kBlock) *
+                           ((d.n + tc::kBlock - 1) / tc::kBlock);
+    const int64_t freqs = ((int64_t)1 << d.lgN) / tc::kFreqs + 1;
+    contract = std::max(contract, blocks * freqs * d.P * (int64_t)sizeof(TcItem));
+  }
+  bytes += contract;
+  if (d.lgN > kMaxLgNOneCta) return bytes;
+  const int64_t per_cta = std::max(1, fwd_team_points() >> d.lgN);
+  for (const int64_t n : {operands, entries}) {
+    const int64_t ctas = (n + per_cta - 1) / per_cta;
+    bytes += ctas * prime_chunks((uint64_t)ctas, d.P, sms) * (int64_t)sizeof(CtaItem);
+  }
+  return bytes;
+}
+
 template <int PLO, int PHI>
 static cudaError_t launch_crt(const InvDesc* descs, const CrtItem* segs, int nsegs,
                               const uint32_t* idx, int count, CrtUniform u, int warp_words,

@@ -119,6 +119,9 @@ constexpr int kCrtMixedSplit = 10;
 void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, double beside,
                uint32_t* nrecs, std::vector<CrtItem>* segs);
 constexpr int kCrtSegLaunches = 2;
+// Most device bytes that the segment records and the work lists of product d
+// (out_words words a result) take in any plan.
+int64_t cut_list_bytes(const ProdDesc& d, uint32_t out_words, int sms);
 cudaError_t launch_crt_mixed(const InvDesc* descs, const CrtItem* segs, int nsegs,
                              const uint32_t* idx, int count, bool high, const int* rmin,
                              const uint32_t* res, uint32_t* out, int32_t* sizes, CrtRec* recs,

@@ -46,8 +46,9 @@ struct Ticket {
 };
 
 // pinned result-size and descriptor staging a slot allocates at start: a
-// batch needs 4 bytes an output entry and about 32 bytes an entry and 12 a
-// contraction block, far below these for any batch under the host-data cap
+// batch needs 4 bytes an output entry, and about 64 bytes an entry and 16 to
+// 24 a contraction block, a transform CTA or a result's segment, far below
+// these for any batch under the host-data cap
 constexpr size_t kStageSizes = (size_t)1 << 20;
 constexpr size_t kStageDescBytes = (size_t)16 << 20;
 
