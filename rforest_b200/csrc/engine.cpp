@@ -677,13 +677,11 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
     if (fixed_b_ && ps.dev_a)
       return set_error(kErrArg, "a plan that keeps B's transforms takes host operands only");
     for (int side = 0; side < 2; ++side) {
-      // one class per product; operands of tensor-core products (blocked
-      // layout) get launches of their own, so the plain kernels stay as
-      // lean, and so do B operands whose transforms the plan keeps
+      // classes by length, primes and digits (each entry's descriptor tells
+      // its layout); B operands whose transforms the plan keeps get launches
+      // of their own
       const bool b_only = fixed_b_ && side == 1;
-      Group& fg =
-          fwdg[{lgN, P * 16 + (r + 29) / 30 + (use_tc ? 1024 : 0) + (b_only ? 2048 : 0)}];
-      fg.tiled = use_tc;
+      Group& fg = fwdg[{lgN, P * 16 + (r + 29) / 30 + (b_only ? 2048 : 0)}];
       fg.b_only = b_only;
       fg.P = P;
       fg.lgN = lgN;
@@ -877,10 +875,9 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
       const bool team = ((int64_t)1 << g.lgN) <= (int64_t)fwd_team_points();
       // a CTA's shared memory follows the launch's largest class, so classes
       // above the team size get launches of their own
-      Group& v = var[{(team ? 0 : g.lgN) + (g.tiled ? 64 : 0) + (g.b_only ? 128 : 0), D}];
+      Group& v = var[{(team ? 0 : g.lgN) + (g.b_only ? 128 : 0), D}];
       v.batched = true;
       v.team = team;
-      v.tiled = g.tiled;
       v.b_only = g.b_only;
       v.D = D;
       if (g.lgN > v.max_lgN) v.max_lgN = g.lgN;

@@ -319,7 +319,6 @@ class Plan {
     bool batched = false;
     bool team = false;
     bool large = false;    // four-step transform (2^lgN above one CTA)
-    bool tiled = false;    // forward: operands of tensor-core products (blocked layout)
     bool b_only = false;   // forward: B operands of a plan that keeps their transforms
     int D = 0;
     int max_lgN = 0;
