@@ -787,7 +787,7 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
         }
     if (!use_tc) cc_prods.push_back(prod_index);
     for (int j = 0; use_tc && j < P; ++j)
-      for (uint64_t h0 = 0; h0 < N; h0 += (uint64_t)kTcFreqsPerCta)
+      for (uint64_t h0 = 0; h0 < N; h0 += (uint64_t)kTcFreqs)
         for (int rb = 0; rb < rbs; ++rb)
           for (int cb = 0; cb < cbs; ++cb) {
             TcItem it;
@@ -862,7 +862,7 @@ int Plan::prepare(std::vector<ProductSpec> prods) {
         out.push_back(std::move(g));
         continue;
       }
-      if (g.lgN < 3 || D > 7) {  // (never a blocked-layout group: lgN >= 3, r <= 192)
+      if (g.lgN < 3) {  // (never a blocked-layout group)
         out.push_back(std::move(g));  // radix-2 path
         continue;
       }

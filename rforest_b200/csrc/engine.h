@@ -205,8 +205,6 @@ inline int tc_bucket_mn(int m, int n) {
   return b < 5 ? b : 4;
 }
 
-constexpr int kTcFreqsPerCta = 128;  // = contract_tc_freqs() (frequencies per tensor-core CTA)
-
 Context& context();
 std::mutex& workspace_mutex();
 

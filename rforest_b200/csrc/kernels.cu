@@ -5,7 +5,7 @@
 //                    residues mod p -> forward NTT, register-blocked passes
 //                    (several small transforms or one large one per CTA)
 //   k_split_fwd      the same, radix 2, one CTA per (entry, prime): tiny
-//                    transforms and digit counts above 7
+//                    transforms (2^2 points)
 //   k_contract       per frequency h and prime: C[h] = A[h] B[h] mod p on
 //                    CUDA cores (64-bit lazy accumulation, Montgomery fold)
 //   k_contract_tc    the same on tensor cores (tcgen05 kind::i8, exact
@@ -2647,7 +2647,7 @@ cudaError_t launch_contract_tc(const ProdDesc* prods, const TcItem* items, int c
   return cudaGetLastError();
 }
 
-int contract_tc_freqs() { return tc::kFreqs; }
+static_assert(kTcFreqs == tc::kFreqs, "work items are cut to the kernel's blocks");
 
 // coefficients a CRT tile can touch for coefficient width rmin
 static int crt_cmax(int P, int rmin) {

@@ -84,7 +84,7 @@ cudaError_t launch_mod_finish(int count, int n, const uint64_t* xl, const int64_
 
 // Tensor-core contraction (tcgen05 kind::i8) for products with m <= 128,
 // k <= 64, n <= 64; shapes: the launch's distinct (m, k, n), nshapes triples
-// (they size its shared memory); each work item covers contract_tc_freqs()
+// (they size its shared memory); each work item covers kTcFreqs
 // consecutive frequencies.  *status is set to 1 if a bounded wait gave up.
 // stall != 0 (failure-path tests only) issues no tensor work, so every CTA's
 // wait runs out.
@@ -99,7 +99,6 @@ cudaError_t launch_check_bounds(const FwdDesc* fwd, int nfwd, const InvDesc* inv
                                 const ProdDesc* prods, int nprods, BoundsCaps caps, int* status,
                                 cudaStream_t st);
 bool contract_tc_eligible(int m, int k, int n);
-int contract_tc_freqs();
 int tc_smem_bytes(int m, int k, int n, int F);
 cudaError_t launch_contract_tc(const ProdDesc* prods, const TcItem* items, int count,
                                uint32_t* res, const int* shapes, int nshapes, int* status,

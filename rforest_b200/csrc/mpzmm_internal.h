@@ -27,7 +27,6 @@ static_assert(kMaxLgN <= kPrimeLgRoot, "transform longer than the primes' 2-powe
 static_assert(kMaxLgN - kLargeLgC <= kTwiddleLg, "four-step columns beyond the table");
 static_assert(2 * 10 == kPrimeLgRoot, "twist exponents are split 10 + 10 bits");
 constexpr int kMaxCoeffBits = 192;  // largest split coefficient (r)
-constexpr int kMaxCrtWords = kMaxPrimes + 1;  // 32-bit words of a CRT value
 
 // Per-prime constants, in __constant__ memory on the device.
 struct PrimeConst {
@@ -52,8 +51,6 @@ struct PrimeConst {
 // 16 products y_j d with y_j < p_j < 2^30 - 2^19, or of 8 with y_j < 2 p_j,
 // fits a signed 64-bit accumulator without carry handling.
 struct CrtConst {
-  uint32_t M[kMaxPrimes + 1][kMaxCrtWords];          // M_P, little-endian words
-  int Mwords[kMaxPrimes + 1];
   // M_P and M_P / p_j, P balanced base-2^30 digits (the last as it comes)
   int32_t M30[kMaxPrimes + 1][kMaxPrimes];
   int32_t mop30[kMaxPrimes + 1][kMaxPrimes][kMaxPrimes];
@@ -90,6 +87,7 @@ struct FwdDesc {
 constexpr int kTcTile = 8;      // frequencies a block of the tensor-core layout (32 bytes)
 constexpr int kTcBlock = 32;    // rows and columns of C a tensor-core work item covers
 constexpr int kTcTileLg = 3;
+constexpr int kTcFreqs = 128;   // frequencies a tensor-core work item covers
 
 // One output polynomial of the inverse transform + CRT + recompose.
 struct InvDesc {

@@ -198,9 +198,7 @@ void build(Moduli& M) {
   std::vector<uint32_t> acc{1};
   for (int P = 1; P <= kMaxPrimes; ++P) {
     mul_small(acc, M.p[P - 1]);
-    int words = (int)acc.size();
-    M.crt.Mwords[P] = words;
-    for (int q = 0; q < words && q < kMaxCrtWords; ++q) M.crt.M[P][q] = acc[q];
+    const int words = (int)acc.size();
     const std::vector<uint32_t> m30 = to_base30(acc);
     balance30(m30, P, M.crt.M30[P]);
     int top = 31;
