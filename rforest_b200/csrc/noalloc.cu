@@ -159,8 +159,10 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
 
   const int P = prm.P, lgN = prm.lgN, r = prm.r;
   const uint64_t N = (uint64_t)1 << lgN, poly = (uint64_t)P * N;
-  // descriptor blob: fwd (A then B), inv, prod; the limits below count 12
-  // bytes for each 128 frequencies of a prime and 4 for each entry besides
+  // descriptor blob: fwd (A then B), inv, prod.  What this entry point takes
+  // is fixed by its documented scratch and by programs sized to it: it counts
+  // 12 bytes for each 128 frequencies of a prime and 4 for each entry besides
+  // the blob, though no list of them is sent.
   const size_t off_fwd = 0;
   const size_t off_inv = align256(off_fwd + sizeof(FwdDesc) * (size_t)(na + nb));
   const size_t off_pd = align256(off_inv + sizeof(InvDesc) * (size_t)nc);
@@ -169,9 +171,13 @@ extern "C" int mpzmm_matmul_noalloc(int m, int k, int n, const uint64_t* d_a_lim
       align256(desc_bytes + 12 * (size_t)P * (size_t)((N + 127) / 128)) +
       sizeof(uint32_t) * (size_t)(na + nb + nc));
   const size_t res_bytes = sizeof(uint32_t) * (size_t)(na + nb + nc) * poly;
-  if (counted > kNoAllocDescBytes || counted + res_bytes > kNoAllocScratchBytes)
+  if (counted > kNoAllocDescBytes)
+    return set_error(kErrTooLarge, "mpzmm_matmul_noalloc: counts " + std::to_string(counted) +
+                                       " bytes of descriptors, the static scratch keeps " +
+                                       std::to_string(kNoAllocDescBytes) + " for them");
+  if (counted + res_bytes > kNoAllocScratchBytes)
     return set_error(kErrTooLarge,
-                     "mpzmm_matmul_noalloc: needs " + std::to_string(counted + res_bytes) +
+                     "mpzmm_matmul_noalloc: counts " + std::to_string(counted + res_bytes) +
                          " scratch bytes, the static scratch holds " +
                          std::to_string(kNoAllocScratchBytes));
 
