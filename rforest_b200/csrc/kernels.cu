@@ -425,7 +425,7 @@ __device__ __forceinline__ uint32_t word_tf(uint32_t y, int g) {
 // (D products of 30-bit by 30-bit numbers, exact in 64 bits for D <= 8), so
 // each prime costs D wide multiply-adds and one Montgomery reduction instead
 // of a Horner chain.  Larger transforms take a whole CTA of 512 or 1024
-// threads, which extracts a coefficient's digits once for kCtaPrimes primes
+// threads, which extracts a coefficient's digits once for cta_primes() primes
 // whose transforms sit in shared memory together.
 //
 // Bound by integer issue: about 58 instructions a residue (2^9 .. 2^11
@@ -1225,7 +1225,7 @@ struct FastDiv {
 
 // The carry into word `wbeg` of a segment, from a look at the 32 words below
 // it (lane l holds word wbeg - 32 + l; lane 0 lacks the word below it, so
-// its own carry stays open): kTfUnknown when every word of 1..31 lets a
+// its own carry stays open): kCarryUnknown when every word of 1..31 lets a
 // carry pass.
 constexpr int kCarryUnknown = 2;
 __device__ __forceinline__ bool tf_const(uint32_t f) {
@@ -1248,7 +1248,7 @@ __device__ __forceinline__ int lookback_carry(uint32_t y, int g, bool prop, int 
 // Words [wbeg, wend) of one output entry by one warp: CRT of its
 // coefficients tile by tile into the warp's scratch sV, each coefficient
 // pre-shifted to its place in the output words (P + 1 words of tile
-// coefficient c at [c (P + 1)]), the words' sums, the carry ripple.
+// coefficient c at [c kCrtStride<P>]), the words' sums, the carry ripple.
 //
 // SEG false: the whole entry (wbeg = 0, wend = out_words), with its sign,
 // negation and size.  SEG true: one segment of an entry that several warps

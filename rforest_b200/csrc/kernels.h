@@ -82,12 +82,6 @@ cudaError_t launch_mod_finish(int count, int n, const uint64_t* xl, const int64_
                               const int32_t* ss, const uint64_t* d, uint64_t* rbuf, int32_t* rs,
                               cudaStream_t st);
 
-// Tensor-core contraction (tcgen05 kind::i8) for products with m <= 128,
-// k <= 64, n <= 64; shapes: the launch's distinct (m, k, n), nshapes triples
-// (they size its shared memory); each work item covers kTcFreqs
-// consecutive frequencies.  *status is set to 1 if a bounded wait gave up.
-// stall != 0 (failure-path tests only) issues no tensor work, so every CTA's
-// wait runs out.
 // Debug check (MPZMM_OPT_CHECK_BOUNDS): every forward, inverse and product
 // descriptor's extents against the workspace capacities (limbs, residue
 // words, output words, result sizes); a thread that finds one outside sets
@@ -98,6 +92,13 @@ struct BoundsCaps {
 cudaError_t launch_check_bounds(const FwdDesc* fwd, int nfwd, const InvDesc* inv, int ninv,
                                 const ProdDesc* prods, int nprods, BoundsCaps caps, int* status,
                                 cudaStream_t st);
+// Tensor-core contraction (tcgen05 kind::i8) for products with m, n <= 1024
+// and k <= 64 (contract_tc_eligible); each work item covers kTcFreqs
+// consecutive frequencies of one block of at most kTcBlock rows and columns
+// of C; shapes: the launch's distinct blocks (rows, k, columns), nshapes
+// triples (they size its shared memory).  *status is set to 1 if a bounded
+// wait gave up.  stall != 0 (failure-path tests only) issues no tensor work,
+// so every CTA's wait runs out.
 bool contract_tc_eligible(int m, int k, int n);
 int tc_smem_bytes(int m, int k, int n, int F);
 cudaError_t launch_contract_tc(const ProdDesc* prods, const TcItem* items, int count,
@@ -105,10 +106,10 @@ cudaError_t launch_contract_tc(const ProdDesc* prods, const TcItem* items, int c
                                cudaStream_t st, int stall = 0);
 
 // CRT + recompose + sign.  crt_items takes the output entries idx and leaves
-// in it those that a warp each recomposes whole, longest first; entries so
-// long that one warp each would leave the GPU (of `sms` SMs) idle go to
-// segs, their records numbered from *nrecs (advanced); launches that run
-// beside this one make its entries `beside` times as many.
+// in it those that a warp each recomposes whole, by prime count and then
+// longest first; entries so long that one warp each would leave the GPU (of
+// `sms` SMs) idle go to segs, their records numbered from *nrecs (advanced);
+// launches that run beside this one make its entries `beside` times as many.
 // launch_crt_mixed runs both lists over several prime counts: high = false
 // takes entries with 2..kCrtMixedSplit primes, high = true those with more;
 // rmin[P] is the narrowest coefficient width among the entries with P primes
