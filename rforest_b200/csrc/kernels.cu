@@ -2679,7 +2679,16 @@ static int crt_segment_words(uint64_t total_words, int sms) {
 // products in 17 chunks were few and cut 350,000 segments, whose lists the
 // host built and the link carried: 11 ms of planning and 559.4 MB to the
 // device, against 7 ms and 550.0 MB.
+//
+// But a chunk waits for its longest entry: one of kCrtLong words takes a warp
+// 0.6 ms, as long as a chunk of 32 MB takes on the link, and few chunks are
+// in flight.  Longer ones are judged by at most kCrtBeside chunks' work: 1000
+// 2 x 2 x 2 products of 2^20 bits host to host 30.8 ms so, 37.2 by the whole
+// batch, 31.3 by each chunk; 512 mixed products 15.4 by the batch, 15.7 by
+// four chunks' work, 16.1 by each chunk.
 constexpr uint32_t kCrtShort = 16 * kCrtTileWords;
+constexpr uint32_t kCrtLong = 28 * 1024;
+constexpr double kCrtBeside = 8.0;
 static uint32_t crt_split(uint32_t W, uint32_t seg, bool few, uint32_t* step) {
   const bool split = few ? W > 2 * seg : W > kCrtShort && W > 6 * seg;
   uint32_t ns = split ? (W + seg - 1) / seg : 1u;
@@ -2713,13 +2722,21 @@ void crt_items(const InvDesc* descs, std::vector<uint32_t>* idx, int sms, double
               (*idx)[i];
   }
   if (!std::is_sorted(keys.begin(), keys.end())) std::sort(keys.begin(), keys.end());
-  const uint32_t seg = (uint32_t)crt_segment_words((uint64_t)((double)total * beside), sms);
-  const bool few = crt_few((uint64_t)((double)keys.size() * beside), sms);
+  const auto segment = [&](double times) {
+    return (uint32_t)crt_segment_words((uint64_t)((double)total * times), sms);
+  };
+  const auto are_few = [&](double times) {
+    return crt_few((uint64_t)((double)keys.size() * times), sms);
+  };
+  const double flight = std::min(beside, kCrtBeside);
+  const uint32_t seg = segment(beside), seg_long = segment(flight);
+  const bool few = are_few(beside), few_long = are_few(flight);
   idx->clear();
   for (const uint64_t key : keys) {
     const uint32_t e = (uint32_t)key, W = descs[e].out_words;
     uint32_t step;
-    const uint32_t ns = crt_split(W, seg, few, &step);
+    const uint32_t ns = W > kCrtLong ? crt_split(W, seg_long, few_long, &step)
+                                     : crt_split(W, seg, few, &step);
     if (ns == 1) {
       idx->push_back(e);
       continue;
